@@ -36,6 +36,7 @@
 #include "hevi_epilogue.cuh"
 #include "hevi_kernels.cuh"
 #include "numfilter_body.cuh"
+#include "rn_div.cuh"
 #include "tma_util.cuh"
 
 namespace hevi {
@@ -53,13 +54,14 @@ template <int S> __host__ __device__ constexpr int box_h() { return TY + 2 * rea
 template <int S> __host__ __device__ constexpr int plane() { return box_k<S>() * box_w<S>() * box_h<S>(); }
 constexpr int NF = 5;                         // staged fields
 enum StagedField : int { F_DN = 0, F_MZ = 1, F_MX = 2, F_MY = 3, F_RT = 4 };
-constexpr int NDP = 33;                       // DPRES levels per column: L0-1 .. L0+31
-constexpr int DP_COLS = (TX + 1) * (TY + 1);  // tile columns and their +x/+y neighbours
+constexpr int NDP = 33;                       // levels of a chunk's level tables: L0-1 .. L0+31
+constexpr int DP_COLS = NCOL + TX + TY;       // DPRES columns: the tile's, then its +x and its +y side
+constexpr int NCARRY = 7;                     // values a column carries into the next chunk
 constexpr int NLT = 6;                        // level tables per chunk: RCDZ, RFDZ, F2H1, F2H2, FDZ, wdamp
 
 template <int S> constexpr size_t smem_bytes()
 {
-    return (size_t)NF * plane<S>() * sizeof(double) + (size_t)(DP_COLS + NCOL + NLT) * NDP * sizeof(double) + 16;
+    return (size_t)NF * plane<S>() * sizeof(double) + (size_t)((DP_COLS + NCOL + NLT) * NDP + NCOL * NCARRY) * sizeof(double) + 16;
 }
 
 struct StateMaps {
@@ -78,20 +80,88 @@ __device__ __forceinline__ R zface_in(R vel, int m, const V &v)
     else return ip4<S>(vel, v(m - 1), v(m), v(m + 1), v(m + 2));
 }
 
-template <int S, typename R, int NM>
-__global__ void __launch_bounds__(32 * NCOL, 2)
-    k_hevi_explicit(const Grid gt, const StageArgsT<R> a, const BatchT<NM> B, const __grid_constant__ StateMaps maps)
+// keeps the compiler from carrying values of the fast path into the rare exact one
+__device__ __forceinline__ void cold() { asm volatile("" ::: "memory"); }
+
+// Where the outputs of a stage go, fixed at compile time so that the marching
+// kernel has no dispatch in its loop: the RkMode itself, with RK_STAGE2 standing
+// for RK_STAGE3 too (they differ in a factor) and FOLD_ANY for the run-time
+// dispatch of put_state/put_flux (Heun's modes).
+constexpr int FOLD_ANY = -1;
+__host__ __device__ constexpr bool fold_reads(int m) { return m == RK_STAGE2 || m == RK_FINAL; }
+
+// The arrays that a thread addresses at its cell, by component: formed on the
+// host, so that an access is one multiply-add on a constant-bank pointer.
+template <typename R>
+struct StagePtrs {
+    const R *nd[15]; // num_diff components q + 5*dir
+    double *acc[5];
+    R *facc[6], *flx[6]; // mflx z, x, y then tflx z, x, y
+    R *Sr, *St, *tZ, *PT;
+};
+
+template <typename R>
+struct StageMaps { // what the host prepares for one launch
+    StagePtrs<R> ptr;
+    StateMaps maps;
+};
+
+template <int M, typename R>
+__device__ __forceinline__ void fold_state(const StageArgsT<R> &a, const StagePtrs<R> &p, size_t N3, int v, double *out,
+                                           const double *x0p, int c, double val, double x0, double acc)
+{
+    if constexpr (M == RK_PLAIN) {
+        sts(out + c, val);
+        flag_nonfinite(a.status, val);
+    } else if constexpr (M == RK_STAGE1) {
+        sts(out + c, val);
+        sts(p.acc[v] + c, val * 2.0);
+    } else if constexpr (M == RK_STAGE2) {
+        sts(out + c, val);
+        sts(p.acc[v] + c, acc + val * (a.rk_mode == RK_STAGE2 ? 4.0 : 2.0));
+    } else if constexpr (M == RK_FINAL) {
+        const double r = rn::sixth((acc + val) - x0 * 3.0);
+        sts(out + c, r);
+        flag_nonfinite(a.status, r);
+    } else {
+        put_state(a, N3, v, out, x0p, (size_t)c, val, true);
+    }
+}
+template <int M, typename R>
+__device__ __forceinline__ void fold_flux(const StageArgsT<R> &a, const StagePtrs<R> &p, size_t N3, int f, int c, R val,
+                                          R acc)
+{
+    if constexpr (M == RK_PLAIN) sts(p.flx[f] + c, val);
+    else if constexpr (M == RK_STAGE1) sts(p.facc[f] + c, val);
+    else if constexpr (M == RK_STAGE2) sts(p.facc[f] + c, acc + val * R(2.0));
+    else if constexpr (M == RK_FINAL) sts(p.flx[f] + c, rn::sixth(acc + val));
+    else put_flux(a, N3, f, (size_t)c, val, true);
+}
+// a flux through the domain's west or south rim, which the combines leave as the last stage's
+template <int M, typename R>
+__device__ __forceinline__ void rim_flux(const StageArgsT<R> &a, const StagePtrs<R> &p, size_t N3, int f, int c, R val)
+{
+    if constexpr (M == RK_PLAIN || M == RK_FINAL) sts(p.flx[f] + c, val);
+    else if constexpr (M == FOLD_ANY) put_flux(a, N3, f, (size_t)c, val, false);
+}
+
+template <int S, typename R, int M, int NM>
+__global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
+    k_hevi_explicit(const Grid gt, const StageArgsT<R> a, const BatchT<NM> B, const StagePtrs<R> ptr,
+                    const __grid_constant__ StateMaps maps)
 {
     constexpr int H = reach<S>(), BW = box_w<S>(), BK = box_k<S>(), PL = plane<S>();
     constexpr int KX = BK, KY = BW * BK; // shared-memory strides of one column step in i and in j
-    constexpr bool W6 = wide_scheme(S);
+    constexpr bool W6 = wide_scheme(S), ACC = fold_reads(M);
     extern __shared__ __align__(1024) double sm[];
     double *stg = sm;                    // NF staged fields, [j][i][k] each
-    double *sdp = sm + NF * PL;          // DPRES, [DP_COLS][NDP]
+    double *sdp = sm + NF * PL;          // DPRES, [DP_COLS][NDP]: levels L0-1 .. L0+31
     double *srp = sdp + DP_COLS * NDP;   // RT2P of the tile's own columns, [NCOL][NDP]
     double *slt = srp + NCOL * NDP;      // the chunk's level tables, [NLT][NDP]
-    uint64_t *bar = reinterpret_cast<uint64_t *>(slt + NLT * NDP);
+    R *scy = reinterpret_cast<R *>(slt + NLT * NDP); // [NCOL][NCARRY]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(slt + NLT * NDP + NCOL * NCARRY);
     __shared__ int s_ok;
+    __shared__ R s_rc[2][NCOL]; // RCDX, RCDY of the columns
 
     int b;
     const Grid g = block_domain(gt, B, b);
@@ -107,21 +177,20 @@ __global__ void __launch_bounds__(32 * NCOL, 2)
         ti = rem / rows;
     }
     const int i0 = g.IS + ti * TX, j0 = g.JS + tj * TY;
-    const int i = i0 + tx, j = j0 + ty;
-    const bool col_ok = i <= g.IE && j <= g.JE;
+    const bool col_ok = i0 + tx <= g.IE && j0 + ty <= g.JE;
+    // warps beyond the domain's edge run along, on its first halo column at most
+    // (whose DPRES the last column needs), and store nothing
+    const int i = min(i0 + tx, g.IE + 1), j = min(j0 + ty, g.JE + 1);
     const size_t N3 = n3(g);
     const int sI = g.KA, sJ = g.KA * g.IA;
     const int KS = g.KS, KE = g.KE;
     const int col = (int)idx3(g, 1, i, j); // offset of level 1 of this warp's column
-    const Nd<R> nd(a, N3);
     const double dt = a.dtrk, J33G = a.J33G;
     const bool use_div = a.divdmp_coef != 0.0;
     const R ddc = use_div ? R(a.divdmp_coef / dt) : R(0.0);
-    const R rcdx = col_ok ? R(ld(g.RCDX + i - 1)) : R(0.0), rcdy = col_ok ? R(ld(g.RCDY + j - 1)) : R(0.0);
     const R h = R(0.5), qr = R(0.25), J33R = R(J33G);
     const unsigned FULL = 0xffffffffu;
     const int NC = (g.KMAX + KC - 1) / KC;
-    R *const sSr = a.colscr, *const sSt = a.colscr + N3, *const stZ = a.colscr + 2 * N3, *const sPT = a.colscr + 3 * N3;
 
     auto issue = [&](int ch) {
         // box origin (0-based): level L0-4 = 32*ch - 2 (even, so its byte offset is a
@@ -132,6 +201,7 @@ __global__ void __launch_bounds__(32 * NCOL, 2)
         for (int f = 0; f < NF; ++f) tma_load_3d(stg + f * PL, &maps.m[f], x, y, z, bar);
     };
     if (tid == 0) {
+        s_ok = 1;
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         issue(0);
@@ -140,37 +210,64 @@ __global__ void __launch_bounds__(32 * NCOL, 2)
 
     // this warp's column in the staged box, at the lane's level of the chunk
     const int cbox = ((ty + H) * BW + (tx + H)) * BK + KLO + lane;
-    const double *sDN = stg + F_DN * PL + cbox, *sMZ = stg + F_MZ * PL + cbox;
-    const double *sMX = stg + F_MX * PL + cbox, *sMY = stg + F_MY * PL + cbox;
-    double *sPO = stg + F_RT * PL + cbox; // RHOT, then POTT
-    // Values of the previous chunk's lane 31 that lane 0 of the next chunk
-    // needs: the fluxes through the face below its level (mass, theta, w, u, v)
-    // and Sr, St one level down. Zero below KS, where every one of them is zero.
-    R Sr_prev = R(0.0), St_prev = R(0.0);
-    R cy_mZ = R(0.0), cy_tZ = R(0.0), cy_qw = R(0.0), cy_qu = R(0.0), cy_qv = R(0.0);
-    double cy_rd = 0.0; // REF_dens one level down
-    // broadcast of lane 31's value (the carry into the next chunk)
-    auto from31 = [&](R v) { return __shfl_sync(FULL, v, 31); };
+    // this column's DPRES and RT2P at level k = L-1 ([1]: at level L), and DPRES at level L
+    // of its +x and +y neighbours: the tile's columns, then the +x and the +y side
+    double *const dpc = sdp + w * NDP + lane, *const rtc = srp + w * NDP + lane;
+    const int dpE = (tx < TX - 1 ? w + 1 : NCOL + ty) * NDP + lane + 1, dpN = (ty < TY - 1 ? w + TX : NCOL + TY + tx) * NDP + lane + 1;
+    // the +x (warps 0..TY-1) or +y (the next TX) side column whose DPRES this warp forms
+    const int ex = w < TY ? TX : w - TY, ey = w < TY ? w : TY;
+    const bool side = w < TX + TY;
+    const int cside = side ? (int)idx3(g, 1, min(i0 + ex, g.IE + 1), min(j0 + ey, g.JE + 1)) : col;
+    // The fluxes through the face below a level (mass, theta, w, u, v), and Sr and St
+    // one level down, are the lane below's: the values are rotated around the warp, and
+    // lane 0, which receives lane 31's, leaves that for the next chunk and takes the
+    // previous chunk's. Zero below KS, where every flux is zero. (In shared memory: as
+    // registers they would spill.)
+    R *const carry = scy + w * NCARRY;
+    if (lane < NCARRY) carry[lane] = R(0.0);
+    if (lane == 0) {
+        s_rc[0][w] = R(ld(g.RCDX + i - 1));
+        s_rc[1][w] = R(ld(g.RCDY + j - 1));
+    }
+    __syncwarp();
+    auto below = [&](R v, int q) {
+        R r = __shfl_sync(FULL, v, (lane + 31) & 31);
+        if (lane == 0) {
+            const R x = carry[q];
+            carry[q] = r;
+            r = x;
+        }
+        return r;
+    };
+    enum { C_MZ, C_TZ, C_SR, C_ST, C_QW, C_QU, C_QV };
 
     for (int ch = 0; ch < NC; ++ch) {
         const int L0 = KS + KC * ch, L = L0 + lane;
-        // ---- the chunk's copies: thread 0 waits (bounded), the block learns the outcome ----
-        if (tid == 0) {
-            const bool ok = mbar_wait(bar, ch & 1);
-            // on a timeout, wait once more (bounded) for the copies still in flight
-            // into this block's shared memory before the block leaves
-            if (!ok) (void)mbar_wait(bar, ch & 1);
-            s_ok = ok ? 1 : 0;
-        }
-        __syncthreads();
-        if (!s_ok) {
-            if (tid == 0) atomicOr(a.status, ST_TMA_TIMEOUT);
-            return; // block-uniform
-        }
-        (void)mbar_try(bar, ch & 1); // completed phase: makes the copied data visible to this thread
+        const int lev = min(L, KE) - 1;  // lanes above KE run along on the last level
+        const int c = col + lev, cs = cside + lev;
+        const bool vb = col_ok && L <= KE;
 
-        // ---- a. the chunk's level tables (levels L0-1..L0+31, clamped to KE), DPRES
-        // of the tile and its +x/+y neighbours (:355) ----
+        // ---- a. DPRES (:355) at the chunk's levels of this warp's column and of its side
+        // column, the level tables (levels L0-1..L0+31, clamped to KE), RHOT -> POTT.
+        // The global operands are on their way before the wait for the copies.
+        const double rt_L = ld(a.RT2P + c), dp0 = ld(a.DPRES0 + c), rr0 = ld(a.REF_rhot + c);
+        double rt_s = 0.0, dp0_s = 0.0, rr_s = 0.0;
+        if (side) { rt_s = ld(a.RT2P + cs); dp0_s = ld(a.DPRES0 + cs); rr_s = ld(a.REF_rhot + cs); }
+        if (!mbar_wait(bar, ch & 1)) { // bounded; the block leaves at the barrier below
+            s_ok = 0;
+            (void)mbar_wait(bar, ch & 1); // bounded: the copies still in flight
+        }
+        double *const sRT = stg + F_RT * PL + cbox;
+        if (lane == 31) { // the previous chunk's last level
+            dpc[-31] = dpc[1];
+            rtc[-31] = rtc[1];
+        }
+        dpc[1] = dp0 + rt_L * (sRT[0] - rr0);
+        rtc[1] = rt_L;
+        if (side) {
+            const double rt = stg[F_RT * PL + ((ey + H) * BW + (ex + H)) * BK + KLO + lane];
+            sdp[(NCOL + w) * NDP + lane + 1] = dp0_s + rt_s * (rt - rr_s);
+        }
         if (w == NCOL - 1) {
             for (int lv = lane; lv < NDP; lv += 32) {
                 const int Lq = min(L0 - 1 + lv, KE);
@@ -182,44 +279,59 @@ __global__ void __launch_bounds__(32 * NCOL, 2)
                 slt[5 * NDP + lv] = ld(a.wdamp + g.z0 + Lq - 1);
             }
         }
-        for (int q = w; q < DP_COLS; q += NCOL) {
-            const int qx = q % (TX + 1), qy = q / (TX + 1);
-            const int ii = i0 + qx, jj = j0 + qy;
-            if (ii > g.IE + 1 || jj > g.JE + 1) continue;
-            const int cq = (int)idx3(g, 1, ii, jj);
-            const double *rt = stg + F_RT * PL + ((qy + H) * BW + (qx + H)) * BK + KLO - 1;
-            for (int lv = lane; lv < NDP; lv += 32) {
-                const int Lq = L0 - 1 + lv;
-                if (Lq > KE) break;
-                const int cc = cq + Lq - 1;
-                const double rt2p = ld(a.RT2P + cc);
-                sdp[q * NDP + lv] = ld(a.DPRES0 + cc) + rt2p * (rt[lv] - ld(a.REF_rhot + cc));
-                if (qx < TX && qy < TY) srp[(qy * TX + qx) * NDP + lv] = rt2p;
+        {
+            // RHOT -> POTT = RHOT/DENS (:586-600) in place, at the levels KS..KE: the tile's own
+            // columns over the whole box height (the vertical stencils), the x/y arms of the
+            // halo at the chunk's levels (the horizontal theta fluxes). A column of the box is
+            // converted by the warp that read its RHOT above.
+            constexpr int NARM = 2 * H * (TX + TY), NPW = NARM / NCOL; // arm columns; per warp
+            static_assert(NARM % NCOL == 0 && TX == TY && TX + TY <= NCOL, "arms per warp");
+            int at[2 + NPW];
+            bool in[2 + NPW];
+            at[0] = cbox - lane - KLO + lane;
+            in[0] = L - KLO >= KS && L - KLO <= KE;
+            at[1] = min(at[0] + 32, cbox - lane - KLO + BK - 1);
+            in[1] = lane < BK - 32 && L - KLO + 32 <= KE;
+#pragma unroll
+            for (int q = 0; q < NPW; ++q) {
+                // arm n: the side column of warp n (n < TX + TY) comes first, so that this warp converts it
+                int bx, by;
+                const int n = q * NCOL + w;
+                if (n < TX + TY) {
+                    bx = ex + H;
+                    by = ey + H;
+                } else {
+                    const int m = n - (TX + TY), d = m / (TX + TY), r = m % (TX + TY); // d: which of the other rings
+                    const int off = d < H ? d : TX + 1 + d;                           // 0..H-1, then TX+H+1..
+                    bx = r < TY ? off : r - TY + H;
+                    by = r < TY ? r + H : off;
+                }
+                at[2 + q] = (by * BW + bx) * BK + KLO + lane;
+                in[2 + q] = L <= KE;
             }
+            rn::Guard<R> gd;
+            R x[2 + NPW], y[2 + NPW];
+#pragma unroll
+            for (int q = 0; q < 2 + NPW; ++q) {
+                x[q] = in[q] ? R(stg[F_RT * PL + at[q]]) : R(0.0);
+                y[q] = in[q] ? R(stg[F_DN * PL + at[q]]) : R(1.0);
+                x[q] = rn::div<true>(gd, x[q], y[q]);
+            }
+            if (gd.bad()) {
+#pragma unroll
+                for (int q = 0; q < 2 + NPW; ++q)
+                    if (in[q]) x[q] = R(stg[F_RT * PL + at[q]]) / R(stg[F_DN * PL + at[q]]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 2 + NPW; ++q)
+                if (in[q]) stg[F_RT * PL + at[q]] = (double)x[q];
         }
         __syncthreads();
-        // RHOT -> POTT = RHOT/DENS (:586-600): the tile's own columns over the whole
-        // box height (the vertical stencils), the x/y arms of the halo at the chunk's
-        // levels (the horizontal theta fluxes)
-        for (int lv = lane; lv < BK; lv += 32) {
-            double *p = sPO - lane - KLO + lv; // box level lv of this warp's column
-            p[0] = (double)(R(p[0]) / R(p[(F_DN - F_RT) * PL]));
+        if (!s_ok) {
+            if (tid == 0) atomicOr(a.status, ST_TMA_TIMEOUT);
+            return; // block-uniform
         }
-        for (int q = w; q < 2 * H * (TX + TY); q += NCOL) {
-            int bx, by;
-            if (q < 2 * H * TY) {
-                const int s = q % (2 * H);
-                by = q / (2 * H) + H;
-                bx = s < H ? s : s + TX;
-            } else {
-                const int q2 = q - 2 * H * TY, s = q2 % (2 * H);
-                bx = q2 / (2 * H) + H;
-                by = s < H ? s : s + TY;
-            }
-            double *p = stg + F_RT * PL + (by * BW + bx) * BK + KLO + lane;
-            p[0] = (double)(R(p[0]) / R(p[(F_DN - F_RT) * PL]));
-        }
-        __syncthreads();
 
         // Chunks clear of the near-wall face forms (every face of the chunk, from
         // the one below L0-1 to the one above L0+31, in the interior range, and
@@ -228,6 +340,8 @@ __global__ void __launch_bounds__(32 * NCOL, 2)
         const bool interior = L0 - 1 >= KS + (W6 ? 2 : 1) && L0 + 31 <= KE - (W6 ? 3 : 2);
         // the level tables at this lane's level L (slot lane+1) and at k = L-1 (slot lane)
         const double *lt = slt + lane;
+#define rcdx s_rc[0][w]
+#define rcdy s_rc[1][w]
 #define rcdz_L lt[0 * NDP + 1]
 #define rfdz_k lt[1 * NDP]
 #define f1_L lt[2 * NDP + 1]
@@ -238,232 +352,256 @@ __global__ void __launch_bounds__(32 * NCOL, 2)
 #define wd_k lt[5 * NDP]
         auto chunk = [&](auto edge) {
             constexpr bool EDGE = decltype(edge)::value;
+            const double *const sDN = stg + F_DN * PL + cbox, *const sMZ = stg + F_MZ * PL + cbox;
+            const double *const sMX = stg + F_MX * PL + cbox, *const sMY = stg + F_MY * PL + cbox;
+            const double *const sPO = stg + F_RT * PL + cbox; // POTT
             auto zf = [&](R vel, int m, const auto &v) -> R {
                 if constexpr (EDGE) return zface<S>(vel, m, KS, KE, v);
                 else return zface_in<S>(vel, m, v);
             };
+            // a value of a column operand at level l, near level m (EDGE: lanes whose
+            // level is out of range evaluate the wall forms at clamped levels, unused)
+            const bool zok = !EDGE || L <= KE - 1; // the face above L carries a flux
             // ---- b. level L: mass and theta fluxes, Sr, St, PT, tZ ----
-            const bool vb = col_ok && (!EDGE || L <= KE);
-            const int c = col + L - 1;
             R Sr = R(0.0), St = R(0.0);
             {
+                const R dz = ld(ptr.nd[0] + c), nTZ = lds(ptr.nd[4] + c);
+                const R nXe = ld(ptr.nd[5] + c), nXw = ld(ptr.nd[5] + c - sI), nYn = ld(ptr.nd[10] + c), nYs = ld(ptr.nd[10] + c - sJ);
+                const R nTXe = ld(ptr.nd[9] + c), nTXw = ld(ptr.nd[9] + c - sI), nTYn = ld(ptr.nd[14] + c), nTYs = ld(ptr.nd[14] + c - sJ);
+                const R tD = lds(a.DENS_t + c), tT = lds(a.RHOT_t + c);
                 // the vertical mass flux through the face above L (hevi_mflx_z :383-391);
-                // the face below is the previous lane's (lane 0: the previous chunk's lane 31)
-                const R mZ = (vb && (!EDGE || L <= KE - 1)) ? ld(nd.DZ() + c) : R(0.0);
-                R mZm1 = __shfl_up_sync(FULL, mZ, 1);
-                if (lane == 0) mZm1 = cy_mZ;
-                cy_mZ = from31(mZ);
+                // the face below is the previous lane's
+                const R mZ = zok ? dz : R(0.0);
+                const R mZm1 = below(mZ, C_MZ);
                 auto P = [&](int l) { return R(sPO[l - L]); };
                 R PT = R(0.0), tZ = R(0.0);
-                if (vb && (!EDGE || L <= KE - 1)) {
+                if (zok) {
                     // PT: valueW_Z (ud3.F90:98-153); tZ: fluxZ_XYZ (ud3.F90:157-247)
                     PT = zf(R(sMZ[0]), L, P);
-                    tZ = mZ * zf(mZ, L, P) + lds(nd.TZ() + c);
+                    tZ = mZ * zf(mZ, L, P) + nTZ;
                 }
-                R tZm = __shfl_up_sync(FULL, tZ, 1);
-                if (lane == 0) tZm = cy_tZ;
-                cy_tZ = from31(tZ);
+                const R tZm = below(tZ, C_TZ);
+                const R Xe = R(sMX[0]) + nXe, Xw = R(sMX[-KX]) + nXw;
+                const R Yn = R(sMY[0]) + nYn, Ys = R(sMY[-KY]) + nYs;
+                const R adv_r = -((Xe - Xw) * rcdx + (Yn - Ys) * rcdy);
+                const R rcdz = R(rcdz_L);
+                Sr = (-(mZ - mZm1) * rcdz + adv_r) + tD;
+                const R aX = ACC ? lds(ptr.facc[1] + c) : R(0.0), aY = ACC ? lds(ptr.facc[2] + c) : R(0.0);
+                const R aTX = ACC ? lds(ptr.facc[4] + c) : R(0.0), aTY = ACC ? lds(ptr.facc[5] + c) : R(0.0);
+                // fluxX/Y_XYZ (ud3.F90:251-353)
+                const R P00 = R(sPO[0]);
+                const R Pm2 = R(sPO[-2 * KX]), Pm1 = R(sPO[-KX]), Pp1 = R(sPO[KX]), Pp2 = R(sPO[2 * KX]);
+                const R Qm2 = R(sPO[-2 * KY]), Qm1 = R(sPO[-KY]), Qp1 = R(sPO[KY]), Qp2 = R(sPO[2 * KY]);
+                const R Pm3 = W6 ? R(sPO[-3 * KX]) : R(0.0), Pp3 = W6 ? R(sPO[3 * KX]) : R(0.0);
+                const R Qm3 = W6 ? R(sPO[-3 * KY]) : R(0.0), Qp3 = W6 ? R(sPO[3 * KY]) : R(0.0);
+                const R tXe = Xe * ip6<S>(Xe, Pm2, Pm1, P00, Pp1, Pp2, Pp3) + nTXe;
+                const R tXw = Xw * ip6<S>(Xw, Pm3, Pm2, Pm1, P00, Pp1, Pp2) + nTXw;
+                const R tYn = Yn * ip6<S>(Yn, Qm2, Qm1, P00, Qp1, Qp2, Qp3) + nTYn;
+                const R tYs = Ys * ip6<S>(Ys, Qm3, Qm2, Qm1, P00, Qp1, Qp2) + nTYs;
+                const R adv_t = -((tXe - tXw) * rcdx + (tYn - tYs) * rcdy); // hevi_st :646-648
+                St = (-(tZ - tZm) * rcdz + adv_t) + tT;                     // hevi_st :646-649
                 if (vb) {
-                    const R Xe = R(sMX[0]) + ld(nd.DX() + c), Xw = R(sMX[-KX]) + ld(nd.DX() + c - sI);
-                    const R Yn = R(sMY[0]) + ld(nd.DY() + c), Ys = R(sMY[-KY]) + ld(nd.DY() + c - sJ);
-                    const R adv_r = -((Xe - Xw) * rcdx + (Yn - Ys) * rcdy);
-                    put_flux(a, N3, 1, c, Xe, true);
-                    put_flux(a, N3, 2, c, Yn, true);
-                    if (i == g.IS) put_flux(a, N3, 1, c - sI, Xw, false);
-                    if (j == g.JS) put_flux(a, N3, 2, c - sJ, Ys, false);
-                    const R rcdz = R(rcdz_L);
-                    Sr = (-(mZ - mZm1) * rcdz + adv_r) + lds(a.DENS_t + c);
-                    // fluxX/Y_XYZ (ud3.F90:251-353)
-                    const R P00 = R(sPO[0]);
-                    const R Pm2 = R(sPO[-2 * KX]), Pm1 = R(sPO[-KX]), Pp1 = R(sPO[KX]), Pp2 = R(sPO[2 * KX]);
-                    const R Qm2 = R(sPO[-2 * KY]), Qm1 = R(sPO[-KY]), Qp1 = R(sPO[KY]), Qp2 = R(sPO[2 * KY]);
-                    const R Pm3 = W6 ? R(sPO[-3 * KX]) : R(0.0), Pp3 = W6 ? R(sPO[3 * KX]) : R(0.0);
-                    const R Qm3 = W6 ? R(sPO[-3 * KY]) : R(0.0), Qp3 = W6 ? R(sPO[3 * KY]) : R(0.0);
-                    const R tXe = Xe * ip6<S>(Xe, Pm2, Pm1, P00, Pp1, Pp2, Pp3) + ld(nd.TX() + c);
-                    const R tXw = Xw * ip6<S>(Xw, Pm3, Pm2, Pm1, P00, Pp1, Pp2) + ld(nd.TX() + c - sI);
-                    const R tYn = Yn * ip6<S>(Yn, Qm2, Qm1, P00, Qp1, Qp2, Qp3) + ld(nd.TY() + c);
-                    const R tYs = Ys * ip6<S>(Ys, Qm3, Qm2, Qm1, P00, Qp1, Qp2) + ld(nd.TY() + c - sJ);
-                    const R adv_t = -((tXe - tXw) * rcdx + (tYn - tYs) * rcdy); // hevi_st :646-648
-                    put_flux(a, N3, 4, c, tXe, true);
-                    put_flux(a, N3, 5, c, tYn, true);
-                    if (i == g.IS) put_flux(a, N3, 4, c - sI, tXw, false);
-                    if (j == g.JS) put_flux(a, N3, 5, c - sJ, tYs, false);
-                    St = (-(tZ - tZm) * rcdz + adv_t) + lds(a.RHOT_t + c); // hevi_st :646-649
-                    sSr[c] = Sr;
-                    sSt[c] = St;
-                    stZ[c] = tZ;
-                    sPT[c] = PT;
+                    fold_flux<M>(a, ptr, N3, 1, c, Xe, aX);
+                    fold_flux<M>(a, ptr, N3, 2, c, Yn, aY);
+                    fold_flux<M>(a, ptr, N3, 4, c, tXe, aTX);
+                    fold_flux<M>(a, ptr, N3, 5, c, tYn, aTY);
+                    if constexpr (M == RK_PLAIN || M == RK_FINAL || M == FOLD_ANY) {
+                        if (i == g.IS) { rim_flux<M>(a, ptr, N3, 1, c - sI, Xw); rim_flux<M>(a, ptr, N3, 4, c - sI, tXw); }
+                        if (j == g.JS) { rim_flux<M>(a, ptr, N3, 2, c - sJ, Ys); rim_flux<M>(a, ptr, N3, 5, c - sJ, tYs); }
+                    }
+                    ptr.Sr[c] = Sr;
+                    ptr.St[c] = St;
+                    ptr.tZ[c] = tZ;
+                    ptr.PT[c] = PT;
                 }
             }
 
             // ---- c. level k = L-1: Sw (hevi_sw :528-578) and C(k) (:698-722) ----
             {
-                R Sr_k = __shfl_up_sync(FULL, Sr, 1), St_k = __shfl_up_sync(FULL, St, 1);
-                if (lane == 0) { Sr_k = Sr_prev; St_k = St_prev; }
-                Sr_prev = from31(Sr);
-                St_prev = from31(St);
+                const int ck = c - 1;
+                const R nZ = lds(ptr.nd[1] + c);
+                const double rd1 = ld(a.REF_dens + c), rd0 = ld(a.REF_dens + ck); // REF_dens(k+1), (k)
+                const R nXe = ld(ptr.nd[6] + ck), nXw = ld(ptr.nd[6] + ck - sI), nYn = ld(ptr.nd[11] + ck), nYs = ld(ptr.nd[11] + ck - sJ);
+                const double W0 = ld(a.MOMZ0 + ck);
+                const R tW = lds(a.MOMZ_t + ck);
+                const R Sr_k = below(Sr, C_SR), St_k = below(St, C_ST);
                 const int k = L - 1;
                 const bool vc = col_ok && (!EDGE || (k >= KS && k <= KE - 1));
                 const double *cMZ = sMZ - 1, *cDN = sDN - 1, *cMX = sMX - 1, *cMY = sMY - 1; // level k
-                const int ck = c - 1;
-                auto vMZ = [&](int l) { return R(cMZ[l - k]); };
-                // vertical w-momentum flux above level k, fluxZ_XYW (ud3.F90:358-452),
-                // zero outside KS..KE-2; the one below is the previous lane's
-                R q_k = R(0.0);
-                if (vc && (!EDGE || k <= KE - 2)) {
-                    const R vel = (R(0.5) * (vMZ(k) + vMZ(k + 1))) / R(cDN[1]);
-                    q_k = J33R * vel * zf(vel, k, vMZ) + lds(nd.WZ() + col + k);
-                }
-                R q_km = __shfl_up_sync(FULL, q_k, 1);
-                if (lane == 0) q_km = cy_qw;
-                cy_qw = from31(q_k);
-                const double rd1 = vb ? lds(a.REF_dens + c) : 0.0; // REF_dens(k+1)
-                double rd0 = __shfl_up_sync(FULL, rd1, 1);         // REF_dens(k)
-                if (lane == 0) rd0 = cy_rd;
-                cy_rd = __shfl_sync(FULL, rd1, 31);
-                if (vc) {
-                    // horizontal w-momentum flux divergence, fluxX/Y_XYW (ud3.F90:598-748)
-                    R adv_w;
-                    {
+                R q_k, adv_w = R(0.0);
+                auto fluxes = [&](auto fast) {
+                    constexpr bool FAST = decltype(fast)::value;
+                    rn::Guard<R> gd;
+                    auto vMZ = [&](int l) { return R(cMZ[l - k]); };
+                    // vertical w-momentum flux above level k, fluxZ_XYW (ud3.F90:358-452),
+                    // zero outside KS..KE-2; the one below is the previous lane's
+                    q_k = R(0.0);
+                    if (!EDGE || (k >= KS && k <= KE - 2)) {
+                        const R vel = rn::div<FAST>(gd, R(0.5) * (vMZ(k) + vMZ(k + 1)), R(cDN[1]));
+                        q_k = J33R * vel * zf(vel, k, vMZ) + nZ;
+                    }
+                    if (!EDGE || (k >= KS && k <= KE - 1)) {
+                        // horizontal w-momentum flux divergence, fluxX/Y_XYW (ud3.F90:598-748)
                         const R f1 = R(f1_k), f2 = R(f2_k);
-                        const R vXe = (f1 * R(cMX[1]) + f2 * R(cMX[0]))
-                                      / (f1 * h * (R(cDN[1]) + R(cDN[1 + KX])) + f2 * h * (R(cDN[0]) + R(cDN[KX])));
-                        const R vXw = (f1 * R(cMX[1 - KX]) + f2 * R(cMX[-KX]))
-                                      / (f1 * h * (R(cDN[1 - KX]) + R(cDN[1])) + f2 * h * (R(cDN[-KX]) + R(cDN[0])));
-                        const R vYn = (f1 * R(cMY[1]) + f2 * R(cMY[0]))
-                                      / (f1 * h * (R(cDN[1]) + R(cDN[1 + KY])) + f2 * h * (R(cDN[0]) + R(cDN[KY])));
-                        const R vYs = (f1 * R(cMY[1 - KY]) + f2 * R(cMY[-KY]))
-                                      / (f1 * h * (R(cDN[1 - KY]) + R(cDN[1])) + f2 * h * (R(cDN[-KY]) + R(cDN[0])));
+                        const R vXe = rn::div<FAST>(gd, f1 * R(cMX[1]) + f2 * R(cMX[0]),
+                                                    f1 * h * (R(cDN[1]) + R(cDN[1 + KX])) + f2 * h * (R(cDN[0]) + R(cDN[KX])));
+                        const R vXw = rn::div<FAST>(gd, f1 * R(cMX[1 - KX]) + f2 * R(cMX[-KX]),
+                                                    f1 * h * (R(cDN[1 - KX]) + R(cDN[1])) + f2 * h * (R(cDN[-KX]) + R(cDN[0])));
+                        const R vYn = rn::div<FAST>(gd, f1 * R(cMY[1]) + f2 * R(cMY[0]),
+                                                    f1 * h * (R(cDN[1]) + R(cDN[1 + KY])) + f2 * h * (R(cDN[0]) + R(cDN[KY])));
+                        const R vYs = rn::div<FAST>(gd, f1 * R(cMY[1 - KY]) + f2 * R(cMY[-KY]),
+                                                    f1 * h * (R(cDN[1 - KY]) + R(cDN[1])) + f2 * h * (R(cDN[-KY]) + R(cDN[0])));
                         const R W_m2 = R(cMZ[-2 * KX]), W_m1 = R(cMZ[-KX]), W_00 = R(cMZ[0]);
                         const R W_p1 = R(cMZ[KX]), W_p2 = R(cMZ[2 * KX]);
                         const R V_m2 = R(cMZ[-2 * KY]), V_m1 = R(cMZ[-KY]), V_p1 = R(cMZ[KY]), V_p2 = R(cMZ[2 * KY]);
                         const R W_m3 = W6 ? R(cMZ[-3 * KX]) : R(0.0), W_p3 = W6 ? R(cMZ[3 * KX]) : R(0.0);
                         const R V_m3 = W6 ? R(cMZ[-3 * KY]) : R(0.0), V_p3 = W6 ? R(cMZ[3 * KY]) : R(0.0);
-                        const R qXe = vXe * ip6<S>(vXe, W_m2, W_m1, W_00, W_p1, W_p2, W_p3) + ld(nd.WX() + ck);
-                        const R qXw = vXw * ip6<S>(vXw, W_m3, W_m2, W_m1, W_00, W_p1, W_p2) + ld(nd.WX() + ck - sI);
-                        const R qYn = vYn * ip6<S>(vYn, V_m2, V_m1, W_00, V_p1, V_p2, V_p3) + ld(nd.WY() + ck);
-                        const R qYs = vYs * ip6<S>(vYs, V_m3, V_m2, V_m1, W_00, V_p1, V_p2) + ld(nd.WY() + ck - sJ);
+                        const R qXe = vXe * ip6<S>(vXe, W_m2, W_m1, W_00, W_p1, W_p2, W_p3) + nXe;
+                        const R qXw = vXw * ip6<S>(vXw, W_m3, W_m2, W_m1, W_00, W_p1, W_p2) + nXw;
+                        const R qYn = vYn * ip6<S>(vYn, V_m2, V_m1, W_00, V_p1, V_p2, V_p3) + nYn;
+                        const R qYs = vYs * ip6<S>(vYs, V_m3, V_m2, V_m1, W_00, V_p1, V_p2) + nYs;
                         adv_w = -((qXe - qXw) * rcdx + (qYn - qYs) * rcdy);
                     }
+                    return gd.bad();
+                };
+                if (fluxes(std::true_type{})) {
+                    cold();
+                    fluxes(std::false_type{});
+                }
+                const R q_km = below(q_k, C_QW);
+                if (vc) {
                     const R advcv = -(q_k - q_km) * R(rfdz_k);
-                    const R wdmp = -R(wd_k) * R(ld(a.MOMZ0 + ck));
+                    const R wdmp = -R(wd_k) * R(W0);
                     const R div = use_div ? ddc * (ld(a.DDIV + ck + 1) - ld(a.DDIV + ck)) * R(fdz_k) : R(0.0);
-                    const R Sw = (advcv + adv_w) + wdmp + div + lds(a.MOMZ_t + ck);
+                    const R Sw = (advcv + adv_w) + wdmp + div + tW;
                     const double rfdz = rfdz_k;
-                    const double *rp = srp + w * NDP + lane; // RT2P at level k
-                    const double RTL1 = rp[1], RTL0 = rp[0];
-                    const double *dp = sdp + (ty * (TX + 1) + tx) * NDP + lane; // DPRES at level k (slot k-L0+1 = lane)
-                    const double pg = -(dp[1] + RTL1 * dt * (double)St - dp[0] - RTL0 * dt * (double)St_k) * rfdz * J33G
+                    const double pg = -(dpc[1] + rtc[1] * dt * (double)St - dpc[0] - rtc[0] * dt * (double)St_k) * rfdz * J33G
                                       - GRAV * (f1_k * (cDN[1] - rd1 + (double)Sr * dt)
                                                 + f2_k * (cDN[0] - rd0 + (double)Sr_k * dt));
-                    a.colC[ck] = cMZ[0] + dt * (pg + (double)Sw);
+                    if (!EDGE || L <= KE) a.colC[ck] = cMZ[0] + dt * (pg + (double)Sw);
                 }
             }
 
             // ---- d. rho*u (hevi_momx :814-928) and rho*v (hevi_momy :934-1048) at level L ----
+            // u
             {
-                const double *dp = sdp + (ty * (TX + 1) + tx) * NDP + lane + 1; // DPRES at level L, this column
-                auto vMX = [&](int l) { return R(sMX[l - L]); };
-                auto vMY = [&](int l) { return R(sMY[l - L]); };
-                const bool do_u = vb && i <= g.IEH, do_v = vb && j <= g.JEH;
-                const bool zok = !EDGE || L <= KE - 1; // the face above L carries a flux
-                // u: the z flux at (u,y,w) above L, fluxZ_UYZ (ud3.F90:753-859); the one
-                // below is the previous lane's
-                {
-                    R q_k = R(0.0);
-                    if (do_u && zok) {
+                const R nZ = lds(ptr.nd[2] + c), nXe = ld(ptr.nd[7] + c + sI), nXw = ld(ptr.nd[7] + c);
+                const R nYn = ld(ptr.nd[12] + c), nYs = ld(ptr.nd[12] + c - sJ), tU = lds(a.MOMX_t + c);
+                const double U0 = lds(a.MOMX0 + c), aU = ACC ? lds(ptr.acc[2] + c) : 0.0;
+                const R fdx = R(ld(g.FDX + i - 1));
+                const double rfdx = ld(g.RFDX + i - 1);
+                const R cor_u = R(0.125) * (R(ld(a.CORIOLI + g.c2 + (i) + (size_t)g.IA * (j - 1)))
+                                            + R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j - 1))));
+                const double dpe = sdp[dpE]; // DPRES at (i+1, j)
+                R q_k, advch;
+                auto fluxes = [&](auto fast) {
+                    constexpr bool FAST = decltype(fast)::value;
+                    rn::Guard<R> gd;
+                    auto vMX = [&](int l) { return R(sMX[l - L]); };
+                    // the z flux at (u,y,w) above L, fluxZ_UYZ (ud3.F90:753-859)
+                    q_k = R(0.0);
+                    if (zok) {
                         const R den = R(f1_L) * h * (R(sDN[1]) + R(sDN[1 + KX]))
                                       + R(f2_L) * h * (R(sDN[0]) + R(sDN[KX]));
-                        const R vel = (h * (R(sMZ[0]) + R(sMZ[KX]))) / den;
-                        q_k = J33R * vel * zf(vel, L, vMX) + lds(nd.UZ() + c);
+                        const R vel = rn::div<FAST>(gd, h * (R(sMZ[0]) + R(sMZ[KX])), den);
+                        q_k = J33R * vel * zf(vel, L, vMX) + nZ;
                     }
-                    R q_km = __shfl_up_sync(FULL, q_k, 1);
-                    if (lane == 0) q_km = cy_qu;
-                    cy_qu = from31(q_k);
-                    if (do_u) {
-                        const R fdx = R(ld(g.FDX + i - 1));
-                        const double rfdx = ld(g.RFDX + i - 1);
-                        const R cor_u = R(0.125) * (R(ld(a.CORIOLI + g.c2 + (i) + (size_t)g.IA * (j - 1)))
-                                                    + R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j - 1))));
-                        const R U_m2 = R(sMX[-2 * KX]), U_m1 = R(sMX[-KX]), U_00 = R(sMX[0]);
-                        const R U_p1 = R(sMX[KX]), U_p2 = R(sMX[2 * KX]);
-                        // x flux at (x,y,z) with the index shift of fluxX_UYZ (ud3.F90:1053-1109)
-                        const R vE = (h * (U_p1 + U_00)) / (R(sDN[KX]));
-                        const R U_m3 = W6 ? R(sMX[-3 * KX]) : R(0.0), U_p3 = W6 ? R(sMX[3 * KX]) : R(0.0);
-                        const R qXe = vE * ip6<S>(vE, U_m2, U_m1, U_00, U_p1, U_p2, U_p3) + ld(nd.UX() + c + sI);
-                        const R vW = (h * (U_00 + U_m1)) / (R(sDN[0]));
-                        const R qXw = vW * ip6<S>(vW, U_m3, U_m2, U_m1, U_00, U_p1, U_p2) + ld(nd.UX() + c);
-                        // y flux at (u,v,z), fluxY_UYZ (ud3.F90:1113-1167)
-                        const R vN = (h * (R(sMY[0]) + R(sMY[KX])))
-                                     / (qr * (R(sDN[0]) + R(sDN[KX]) + R(sDN[KY]) + R(sDN[KX + KY])));
-                        const R qYn = vN * ip6<S>(vN, W6 ? R(sMX[-2 * KY]) : R(0.0), R(sMX[-KY]), U_00, R(sMX[KY]),
-                                                  R(sMX[2 * KY]), W6 ? R(sMX[3 * KY]) : R(0.0)) + ld(nd.UY() + c);
-                        const R vS = (h * (R(sMY[-KY]) + R(sMY[KX - KY])))
-                                     / (qr * (R(sDN[-KY]) + R(sDN[KX - KY]) + R(sDN[0]) + R(sDN[KX])));
-                        const R qYs = vS * ip6<S>(vS, W6 ? R(sMX[-3 * KY]) : R(0.0), R(sMX[-2 * KY]), R(sMX[-KY]), U_00,
-                                                  R(sMX[KY]), W6 ? R(sMX[2 * KY]) : R(0.0)) + ld(nd.UY() + c - sJ);
-                        const R advcv = -(q_k - q_km) * R(rcdz_L);
-                        const R advch = -((qXe - qXw) * R(rfdx) + (qYn - qYs) * rcdy);
-                        const double DPe = dp[NDP]; // DPRES at (i+1, j)
-                        const double pg = (DPe - dp[0]) * rfdx;
-                        const R cf = cor_u * (R(sMY[KX]) + R(sMY[0]) + R(sMY[KX - KY]) + R(sMY[-KY]));
-                        const R div = !use_div ? R(0.0) : ddc * (ld(a.DDIV + c + sI) - ld(a.DDIV + c)) * fdx;
-                        const double val = lds(a.MOMX0 + c)
-                                           + dt * (((((double)(advcv + advch)) - pg) + (double)cf) + (double)div
-                                                   + (double)lds(a.MOMX_t + c));
-                        put_state(a, N3, 2, a.MOMX_RK, a.MOMX0, c, val, true);
-                    }
+                    const R U_m2 = R(sMX[-2 * KX]), U_m1 = R(sMX[-KX]), U_00 = R(sMX[0]);
+                    const R U_p1 = R(sMX[KX]), U_p2 = R(sMX[2 * KX]);
+                    // x flux at (x,y,z) with the index shift of fluxX_UYZ (ud3.F90:1053-1109)
+                    const R vE = rn::div<FAST>(gd, h * (U_p1 + U_00), R(sDN[KX]));
+                    const R vW = rn::div<FAST>(gd, h * (U_00 + U_m1), R(sDN[0]));
+                    // y flux at (u,v,z), fluxY_UYZ (ud3.F90:1113-1167)
+                    const R vN = rn::div<FAST>(gd, h * (R(sMY[0]) + R(sMY[KX])),
+                                               qr * (R(sDN[0]) + R(sDN[KX]) + R(sDN[KY]) + R(sDN[KX + KY])));
+                    const R vS = rn::div<FAST>(gd, h * (R(sMY[-KY]) + R(sMY[KX - KY])),
+                                               qr * (R(sDN[-KY]) + R(sDN[KX - KY]) + R(sDN[0]) + R(sDN[KX])));
+                    const R U_m3 = W6 ? R(sMX[-3 * KX]) : R(0.0), U_p3 = W6 ? R(sMX[3 * KX]) : R(0.0);
+                    const R qXe = vE * ip6<S>(vE, U_m2, U_m1, U_00, U_p1, U_p2, U_p3) + nXe;
+                    const R qXw = vW * ip6<S>(vW, U_m3, U_m2, U_m1, U_00, U_p1, U_p2) + nXw;
+                    const R qYn = vN * ip6<S>(vN, W6 ? R(sMX[-2 * KY]) : R(0.0), R(sMX[-KY]), U_00, R(sMX[KY]),
+                                              R(sMX[2 * KY]), W6 ? R(sMX[3 * KY]) : R(0.0)) + nYn;
+                    const R qYs = vS * ip6<S>(vS, W6 ? R(sMX[-3 * KY]) : R(0.0), R(sMX[-2 * KY]), R(sMX[-KY]), U_00,
+                                              R(sMX[KY]), W6 ? R(sMX[2 * KY]) : R(0.0)) + nYs;
+                    advch = -((qXe - qXw) * R(rfdx) + (qYn - qYs) * rcdy);
+                    return gd.bad() && vb;
+                };
+                if (fluxes(std::true_type{})) {
+                    cold();
+                    fluxes(std::false_type{});
                 }
-                // v: the z flux at (x,v,w), fluxZ_XVZ (ud3.F90:1173-1279)
-                {
-                    R q_k = R(0.0);
-                    if (do_v && zok) {
+                const R q_km = below(q_k, C_QU);
+                if (vb && i <= g.IEH) {
+                    const R advcv = -(q_k - q_km) * R(rcdz_L);
+                    const double pg = (dpe - dpc[1]) * rfdx;
+                    const R cf = cor_u * (R(sMY[KX]) + R(sMY[0]) + R(sMY[KX - KY]) + R(sMY[-KY]));
+                    const R div = !use_div ? R(0.0) : ddc * (ld(a.DDIV + c + sI) - ld(a.DDIV + c)) * fdx;
+                    const double val = U0 + dt * (((((double)(advcv + advch)) - pg) + (double)cf) + (double)div + (double)tU);
+                    fold_state<M>(a, ptr, N3, 2, a.MOMX_RK, a.MOMX0, c, val, U0, aU);
+                }
+            }
+            // v
+            {
+                const R nZ = lds(ptr.nd[3] + c), nXe = ld(ptr.nd[8] + c), nXw = ld(ptr.nd[8] + c - sI);
+                const R nYn = ld(ptr.nd[13] + c + sJ), nYs = ld(ptr.nd[13] + c), tV = lds(a.MOMY_t + c);
+                const double V0 = lds(a.MOMY0 + c), aV = ACC ? lds(ptr.acc[3] + c) : 0.0;
+                const R fdy = R(ld(g.FDY + j - 1));
+                const double rfdy = ld(g.RFDY + j - 1);
+                const R cor_v = R(-0.125) * (R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j)))
+                                             + R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j - 1))));
+                const double dpn = sdp[dpN]; // DPRES at (i, j+1)
+                R q_k, advch;
+                auto fluxes = [&](auto fast) {
+                    constexpr bool FAST = decltype(fast)::value;
+                    rn::Guard<R> gd;
+                    auto vMY = [&](int l) { return R(sMY[l - L]); };
+                    // the z flux at (x,v,w), fluxZ_XVZ (ud3.F90:1173-1279)
+                    q_k = R(0.0);
+                    if (zok) {
                         const R den = R(f1_L) * h * (R(sDN[1]) + R(sDN[1 + KY]))
                                       + R(f2_L) * h * (R(sDN[0]) + R(sDN[KY]));
-                        const R vel = (h * (R(sMZ[0]) + R(sMZ[KY]))) / den;
-                        q_k = J33R * vel * zf(vel, L, vMY) + lds(nd.VZ() + c);
+                        const R vel = rn::div<FAST>(gd, h * (R(sMZ[0]) + R(sMZ[KY])), den);
+                        q_k = J33R * vel * zf(vel, L, vMY) + nZ;
                     }
-                    R q_km = __shfl_up_sync(FULL, q_k, 1);
-                    if (lane == 0) q_km = cy_qv;
-                    cy_qv = from31(q_k);
-                    if (do_v) {
-                        const R fdy = R(ld(g.FDY + j - 1));
-                        const double rfdy = ld(g.RFDY + j - 1);
-                        const R cor_v = R(-0.125) * (R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j)))
-                                                     + R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j - 1))));
-                        const R Y_m2 = R(sMY[-2 * KY]), Y_m1 = R(sMY[-KY]), Y_00 = R(sMY[0]);
-                        const R Y_p1 = R(sMY[KY]), Y_p2 = R(sMY[2 * KY]);
-                        // x flux at (u,v,z), fluxX_XVZ (ud3.F90:1473-1527)
-                        const R vE = (h * (R(sMX[0]) + R(sMX[KY])))
-                                     / (qr * (R(sDN[0]) + R(sDN[KX]) + R(sDN[KY]) + R(sDN[KX + KY])));
-                        const R qXe = vE * ip6<S>(vE, W6 ? R(sMY[-2 * KX]) : R(0.0), R(sMY[-KX]), Y_00, R(sMY[KX]),
-                                                  R(sMY[2 * KX]), W6 ? R(sMY[3 * KX]) : R(0.0)) + ld(nd.VX() + c);
-                        const R vW = (h * (R(sMX[-KX]) + R(sMX[KY - KX])))
-                                     / (qr * (R(sDN[-KX]) + R(sDN[0]) + R(sDN[KY - KX]) + R(sDN[KY])));
-                        const R qXw = vW * ip6<S>(vW, W6 ? R(sMY[-3 * KX]) : R(0.0), R(sMY[-2 * KX]), R(sMY[-KX]), Y_00,
-                                                  R(sMY[KX]), W6 ? R(sMY[2 * KX]) : R(0.0)) + ld(nd.VX() + c - sI);
-                        // y flux with the index shift of fluxY_XVZ (ud3.F90:1531-1587)
-                        const R vN = (h * (Y_p1 + Y_00)) / (R(sDN[KY]));
-                        const R Y_m3 = W6 ? R(sMY[-3 * KY]) : R(0.0), Y_p3 = W6 ? R(sMY[3 * KY]) : R(0.0);
-                        const R qYn = vN * ip6<S>(vN, Y_m2, Y_m1, Y_00, Y_p1, Y_p2, Y_p3) + ld(nd.VY() + c + sJ);
-                        const R vS = (h * (Y_00 + Y_m1)) / (R(sDN[0]));
-                        const R qYs = vS * ip6<S>(vS, Y_m3, Y_m2, Y_m1, Y_00, Y_p1, Y_p2) + ld(nd.VY() + c);
-                        const R advcv = -(q_k - q_km) * R(rcdz_L);
-                        const R advch = -((qXe - qXw) * rcdx + (qYn - qYs) * R(rfdy));
-                        const double DPn = dp[(TX + 1) * NDP]; // DPRES at (i, j+1)
-                        const double pg = (DPn - dp[0]) * rfdy;
-                        const R cf = cor_v * (R(sMX[KY]) + R(sMX[0]) + R(sMX[KY - KX]) + R(sMX[-KX]));
-                        const R div = !use_div ? R(0.0) : ddc * (ld(a.DDIV + c + sJ) - ld(a.DDIV + c)) * fdy;
-                        const double val = lds(a.MOMY0 + c)
-                                           + dt * (((((double)(advcv + advch)) - pg) + (double)cf) + (double)div
-                                                   + (double)lds(a.MOMY_t + c));
-                        put_state(a, N3, 3, a.MOMY_RK, a.MOMY0, c, val, true);
-                    }
+                    const R Y_m2 = R(sMY[-2 * KY]), Y_m1 = R(sMY[-KY]), Y_00 = R(sMY[0]);
+                    const R Y_p1 = R(sMY[KY]), Y_p2 = R(sMY[2 * KY]);
+                    // x flux at (u,v,z), fluxX_XVZ (ud3.F90:1473-1527)
+                    const R vE = rn::div<FAST>(gd, h * (R(sMX[0]) + R(sMX[KY])),
+                                               qr * (R(sDN[0]) + R(sDN[KX]) + R(sDN[KY]) + R(sDN[KX + KY])));
+                    const R vW = rn::div<FAST>(gd, h * (R(sMX[-KX]) + R(sMX[KY - KX])),
+                                               qr * (R(sDN[-KX]) + R(sDN[0]) + R(sDN[KY - KX]) + R(sDN[KY])));
+                    // y flux with the index shift of fluxY_XVZ (ud3.F90:1531-1587)
+                    const R vN = rn::div<FAST>(gd, h * (Y_p1 + Y_00), R(sDN[KY]));
+                    const R vS = rn::div<FAST>(gd, h * (Y_00 + Y_m1), R(sDN[0]));
+                    const R qXe = vE * ip6<S>(vE, W6 ? R(sMY[-2 * KX]) : R(0.0), R(sMY[-KX]), Y_00, R(sMY[KX]),
+                                              R(sMY[2 * KX]), W6 ? R(sMY[3 * KX]) : R(0.0)) + nXe;
+                    const R qXw = vW * ip6<S>(vW, W6 ? R(sMY[-3 * KX]) : R(0.0), R(sMY[-2 * KX]), R(sMY[-KX]), Y_00,
+                                              R(sMY[KX]), W6 ? R(sMY[2 * KX]) : R(0.0)) + nXw;
+                    const R Y_m3 = W6 ? R(sMY[-3 * KY]) : R(0.0), Y_p3 = W6 ? R(sMY[3 * KY]) : R(0.0);
+                    const R qYn = vN * ip6<S>(vN, Y_m2, Y_m1, Y_00, Y_p1, Y_p2, Y_p3) + nYn;
+                    const R qYs = vS * ip6<S>(vS, Y_m3, Y_m2, Y_m1, Y_00, Y_p1, Y_p2) + nYs;
+                    advch = -((qXe - qXw) * rcdx + (qYn - qYs) * R(rfdy));
+                    return gd.bad() && vb;
+                };
+                if (fluxes(std::true_type{})) {
+                    cold();
+                    fluxes(std::false_type{});
+                }
+                const R q_km = below(q_k, C_QV);
+                if (vb && j <= g.JEH) {
+                    const R advcv = -(q_k - q_km) * R(rcdz_L);
+                    const double pg = (dpn - dpc[1]) * rfdy;
+                    const R cf = cor_v * (R(sMX[KY]) + R(sMX[0]) + R(sMX[KY - KX]) + R(sMX[-KX]));
+                    const R div = !use_div ? R(0.0) : ddc * (ld(a.DDIV + c + sJ) - ld(a.DDIV + c)) * fdy;
+                    const double val = V0 + dt * (((((double)(advcv + advch)) - pg) + (double)cf) + (double)div + (double)tV);
+                    fold_state<M>(a, ptr, N3, 3, a.MOMY_RK, a.MOMY0, c, val, V0, aV);
                 }
             }
         };
         if (interior) chunk(std::false_type{});
         else chunk(std::true_type{});
+#undef rcdx
+#undef rcdy
 #undef rcdz_L
 #undef rfdz_k
 #undef f1_L
@@ -481,86 +619,135 @@ __global__ void __launch_bounds__(32 * NCOL, 2)
 // =============================================================================
 // k_hevi_column: the column problem of CCOLS columns per CTA
 // =============================================================================
-// The CTA loads C, PT and A(k) of its columns into shared memory, and the
-// per-level factors B(k) and RFDZ(k) of the coefficients once for all of
-// them. Warp 0 runs the Thomas solve (solve_direct :1092-1127) one lane per
-// column: the coefficients of level k+1 are formed while the division of
-// level k runs, so that only e(k-1) and f(k-1) chain the levels. Then all warps
-// back-update rho, rho*w, rho*theta and the vertical fluxes (:728-790).
+// The CTA copies C, PT and RT2P of its columns into shared memory with
+// cp.async, every copy in flight at once, and forms the per-level factors of the
+// coefficients once for all columns. Warp 0 runs the Thomas solve
+// (solve_direct :1092-1127) one lane per column: the coefficients of level k+1
+// are formed while the division of level k runs, so that only e(k-1) and f(k-1)
+// chain the levels. The other warps meanwhile load the operands of their first
+// part of the back-update of rho, rho*w, rho*theta and the vertical fluxes
+// (:728-790), which all warps then run, a column's 32 levels at a time.
 constexpr int CCOLS = 16;  // columns per CTA (consecutive in i)
 constexpr int CWARPS = 8;
 __host__ __device__ inline int col_pitch_c(int KA) { return KA | 1; }
-__host__ __device__ inline size_t column_smem(int KA) { return ((size_t)3 * CCOLS * col_pitch_c(KA) + 2 * (size_t)KA) * sizeof(double); }
+__host__ __device__ inline size_t column_smem(int KA) { return ((size_t)3 * CCOLS * col_pitch_c(KA) + 3 * (size_t)KA) * sizeof(double); }
 
-template <typename R, int NM>
-__global__ void __launch_bounds__(32 * CWARPS, 4) k_hevi_column(const Grid gt, const StageArgsT<R> a, const BatchT<NM> B)
+// asynchronous copy of one value into shared memory, from this thread's view
+// complete after copy_wait
+template <typename T>
+__device__ __forceinline__ void copy_async(T *dst, const T *src)
 {
+    static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async sizes");
+    if constexpr (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <typename R, int M, int NM>
+__global__ void __launch_bounds__(32 * CWARPS, 4)
+    k_hevi_column(const Grid gt, const StageArgsT<R> a, const BatchT<NM> B, const StagePtrs<R> ptr)
+{
+    constexpr bool ACC = fold_reads(M);
     extern __shared__ double csm[];
     int b;
     const Grid g = block_domain(gt, B, b);
     const int nbx = (g.IMAX + CCOLS - 1) / CCOLS;
     const int i0 = g.IS + (b % nbx) * CCOLS, j = g.JS + b / nbx;
+    const int ncol = min(CCOLS, g.IE - i0 + 1);
     const int lane = threadIdx.x, w = threadIdx.y;
     const size_t N3 = n3(g);
-    const int KS = g.KS, KE = g.KE, KP = col_pitch_c(g.KA);
+    const int KS = g.KS, KE = g.KE, KP = col_pitch_c(g.KA), NP = (g.KMAX + 31) / 32;
     const double dt = a.dtrk, J33G = a.J33G, dt2 = dt * dt;
-    const Nd<R> nd(a, N3);
-    const R *sSr = a.colscr, *sSt = a.colscr + N3, *stZ = a.colscr + 2 * N3, *sPT = a.colscr + 3 * N3;
+    const int col0 = (int)idx3(g, 1, i0, j);
     // per-level arrays of the tile's columns: [array][column][level], odd pitch;
-    // then B(k) and RFDZ(k) by level
-    double *sC = csm, *sP = csm + (size_t)CCOLS * KP, *sA = csm + (size_t)2 * CCOLS * KP;
-    double *sB = csm + (size_t)3 * CCOLS * KP, *sR = sB + g.KA;
-#define CA(arr, cc, L) arr[(size_t)(cc) * KP + (L) - 1]
+    // then dt^2 J33G RCDZ, B and RFDZ by level
+    double *sC = csm, *sA = csm + (size_t)CCOLS * KP;
+    R *sP = reinterpret_cast<R *>(csm + (size_t)2 * CCOLS * KP);
+    double *sD = csm + (size_t)3 * CCOLS * KP, *sB = sD + g.KA, *sR = sB + g.KA;
+#define CA(arr, cc, L) arr[(cc) * KP + (L) - 1]
 
-    // ---- load C, PT and A(k) = dt^2 J33G^2 RCDZ RT2P (:696); B(k) (:697) and RFDZ(k) ----
-    for (int cc = w; cc < CCOLS; cc += CWARPS) {
-        const int i = i0 + cc;
-        if (i > g.IE) break;
-        const int col = (int)idx3(g, 1, i, j);
+    // ---- C, PT and RT2P of the columns; the level factors of A(k) (:696), B(k) (:697), RFDZ(k) ----
+    for (int cc = w; cc < ncol; cc += CWARPS) {
+        const int col = col0 + cc * g.KA;
         for (int L = KS + lane; L <= KE; L += 32) {
             const int c = col + L - 1;
             if (L <= KE - 1) {
-                CA(sC, cc, L) = __ldcg(a.colC + c);
-                CA(sP, cc, L) = (double)__ldcg(sPT + c);
+                copy_async(&CA(sC, cc, L), (const double *)a.colC + c);
+                copy_async(&CA(sP, cc, L), (const R *)ptr.PT + c);
             }
-            CA(sA, cc, L) = dt2 * J33G * ld(g.RCDZ + L - 1) * ld(a.RT2P + c) * J33G;
+            copy_async(&CA(sA, cc, L), a.RT2P + c);
         }
     }
-    for (int k = KS + w * 32 + lane; k <= KE - 1; k += 32 * CWARPS) {
-        sB[k - 1] = GRAV * dt2 * J33G / (ld(g.CDZ + k) + ld(g.CDZ + k - 1));
-        sR[k - 1] = ld(g.RFDZ + k - 1);
+    for (int k = KS + w * 32 + lane; k <= KE; k += 32 * CWARPS) {
+        sD[k - 1] = dt2 * J33G * ld(g.RCDZ + k - 1);
+        if (k <= KE - 1) {
+            sB[k - 1] = GRAV * dt2 * J33G / (ld(g.CDZ + k) + ld(g.CDZ + k - 1));
+            sR[k - 1] = ld(g.RFDZ + k - 1);
+        }
     }
+
+    // operands of the back-update of one column's 32 levels
+    struct Ops {
+        double D0, T0, W0, W, aD, aT, aW;
+        R Sr, St, tZ, nDZ, aM, aQ;
+    };
+    auto load_ops = [&](int item, Ops &o) {
+        const int m = min(KS + (item / CCOLS) * 32 + lane, KE), cc = min(item % CCOLS, ncol - 1);
+        const int c = col0 + cc * g.KA + m - 1;
+        o.Sr = __ldcg(ptr.Sr + c); o.St = __ldcg(ptr.St + c); o.tZ = __ldcg(ptr.tZ + c);
+        o.nDZ = ld(ptr.nd[0] + c);
+        o.D0 = lds(a.DENS0 + c); o.T0 = lds(a.RHOT0 + c); o.W0 = ld(a.MOMZ0 + c); o.W = ld(a.MOMZ + c);
+        if constexpr (ACC) {
+            o.aD = lds(ptr.acc[0] + c); o.aT = lds(ptr.acc[4] + c); o.aW = lds(ptr.acc[1] + c);
+            o.aM = lds(ptr.facc[0] + c); o.aQ = lds(ptr.facc[3] + c);
+        }
+    };
+    Ops o{};
+    copy_wait();
     __syncthreads();
+    if (w > 0) load_ops(w, o);
 
     // ---- Thomas solve, one lane per column (F1..F3 of :699-709) ----
-    if (w == 0 && lane < CCOLS && i0 + lane <= g.IE) {
+    if (w == 0 && lane < ncol) {
         const int cc = lane;
-        // F1, F2, F3 and C of level k (F1 is not used at KE-1, F3 not at KS)
-        auto coef = [&](int k, double &F1, double &F2, double &F3, double &Ck) {
+        // A(k) = dt^2 J33G^2 RCDZ RT2P (:696)
+        auto Ak = [&](int k) { return sD[k - 1] * CA(sA, cc, k) * J33G; };
+        auto Pk = [&](int k) { return (double)CA(sP, cc, k); };
+        // F1, F2, F3 and C of level k (F1 is not used at KE-1, F3 not at KS) with A(k), A(k+1)
+        // and PT(k-1), PT(k), PT(k+1)
+        auto coef = [&](int k, double A0, double A1, double Pm, double P0, double Pp, double &F1, double &F2, double &F3,
+                        double &Ck) {
             const double rfdz = sR[k - 1], Bk = sB[k - 1];
-            const double Ak = CA(sA, cc, k), Ak1 = CA(sA, cc, k + 1);
-            F2 = 1.0 + (CA(sP, cc, k) * rfdz * (Ak1 + Ak));
-            F1 = k <= KE - 2 ? -(CA(sP, cc, k + 1) * rfdz * Ak1 + Bk) : 0.0;
-            F3 = k >= KS + 1 ? -(CA(sP, cc, k - 1) * rfdz * Ak - Bk) : 0.0;
+            F2 = 1.0 + (P0 * rfdz * (A1 + A0));
+            F1 = -(Pp * rfdz * A1 + Bk);
+            F3 = -(Pm * rfdz * A0 - Bk);
             Ck = CA(sC, cc, k);
         };
+        // A0 = A(k+1), A1 = A(k+2); Pm, P0, Pp = PT(k), PT(k+1), PT(k+2) of the level k being solved
+        double Pm = 0.0, P0 = Pk(KS), Pp = Pk(KS + 1), A0 = Ak(KS), A1 = Ak(KS + 1);
         double F1, F2, F3, Ck;
-        coef(KS, F1, F2, F3, Ck);
+        coef(KS, A0, A1, Pm, P0, Pp, F1, F2, F3, Ck);
         double e_prev, f_prev;
         {
             const double rdenom = 1.0 / F2;
             e_prev = -F1 * rdenom;
             f_prev = Ck * rdenom;
         }
+        auto up = [&](int k) { // the operands of level k
+            Pm = P0; P0 = Pp; Pp = k <= KE - 2 ? Pk(k + 1) : 0.0;
+            A0 = A1; A1 = Ak(k + 1);
+        };
         double nF1, nF2, nF3, nC; // the next level's coefficients
-        coef(KS + 1, nF1, nF2, nF3, nC);
+        up(KS + 1);
+        coef(KS + 1, A0, A1, Pm, P0, Pp, nF1, nF2, nF3, nC);
         // levels KS+1..KE-2: one straight block per level, in which the next
         // level's coefficients fill the latency of this level's division
         for (int k = KS + 1; k <= KE - 2; ++k) {
             F1 = nF1; F2 = nF2; F3 = nF3; Ck = nC;
+            up(k + 1); // reads RT2P(k+2): not yet overwritten
             CA(sA, cc, k - 1) = e_prev;
             CA(sC, cc, k - 1) = f_prev;
-            coef(k + 1, nF1, nF2, nF3, nC); // reads A(k+1), A(k+2): not yet overwritten
+            coef(k + 1, A0, A1, Pm, P0, Pp, nF1, nF2, nF3, nC);
             const double rdenom = 1.0 / (F2 + F3 * e_prev);
             e_prev = -F1 * rdenom;
             f_prev = (Ck - F3 * f_prev) * rdenom;
@@ -572,6 +759,7 @@ __global__ void __launch_bounds__(32 * CWARPS, 4) k_hevi_column(const Grid gt, c
         CA(sC, cc, KE - 1) = f_prev;
         // back substitution, C(k) = e(k) C(k+1) + f(k)
         double Cnext = f_prev;
+#pragma unroll 4
         for (int k = KE - 2; k >= KS; --k) {
             Cnext = CA(sA, cc, k) * Cnext + CA(sC, cc, k);
             CA(sC, cc, k) = Cnext;
@@ -580,52 +768,51 @@ __global__ void __launch_bounds__(32 * CWARPS, 4) k_hevi_column(const Grid gt, c
     __syncthreads();
 
     // ---- back-update (:728-790) ----
-    for (int cc = w; cc < CCOLS; cc += CWARPS) {
-        const int i = i0 + cc;
-        if (i > g.IE) break;
-        const int col = (int)idx3(g, 1, i, j);
-        for (int m = KS + lane; m <= KE; m += 32) {
-            const int c = col + m - 1;
+    for (int item = w; item < CCOLS * NP; item += CWARPS) {
+        if (item != w || w == 0) load_ops(item, o);
+        const int cc = item % CCOLS, i = i0 + cc;
+        const int m = KS + (item / CCOLS) * 32 + lane;
+        const int c = col0 + cc * g.KA + m - 1;
+        if (cc >= ncol) continue;
+        if (m <= KE) {
             const double rcdz = ld(g.RCDZ + m - 1);
+            const double Cm = m <= KE - 1 ? CA(sC, cc, m) : 0.0, Cm1 = m >= KS + 1 ? CA(sC, cc, m - 1) : 0.0;
+            const double Pm = m <= KE - 1 ? (double)CA(sP, cc, m) : 0.0, Pm1 = m >= KS + 1 ? (double)CA(sP, cc, m - 1) : 0.0;
             double adr, adt;
             if (m == KE) {
-                const double Cm1 = CA(sC, cc, m - 1);
                 adr = Cm1 * J33G * rcdz;
-                adt = Cm1 * CA(sP, cc, KE - 1) * J33G * rcdz;
+                adt = Cm1 * Pm1 * J33G * rcdz;
             } else if (m == KS) {
-                const double Cm = CA(sC, cc, m);
                 adr = -Cm * J33G * rcdz;
-                adt = -Cm * CA(sP, cc, KS) * J33G * rcdz;
+                adt = -Cm * Pm * J33G * rcdz;
             } else {
-                const double Cm = CA(sC, cc, m), Cm1 = CA(sC, cc, m - 1);
                 adr = -(Cm - Cm1) * J33G * rcdz;
-                adt = -(Cm * CA(sP, cc, m) - Cm1 * CA(sP, cc, m - 1)) * J33G * rcdz;
+                adt = -(Cm * Pm - Cm1 * Pm1) * J33G * rcdz;
             }
-            put_state(a, N3, 0, a.DENS_RK, a.DENS0, c, lds(a.DENS0 + c) + dt * (adr + (double)__ldcg(sSr + c)), true);
-            put_state(a, N3, 4, a.RHOT_RK, a.RHOT0, c, lds(a.RHOT0 + c) + dt * (adt + (double)__ldcg(sSt + c)), true);
+            fold_state<M>(a, ptr, N3, 0, a.DENS_RK, a.DENS0, c, o.D0 + dt * (adr + (double)o.Sr), o.D0, o.aD);
+            fold_state<M>(a, ptr, N3, 4, a.RHOT_RK, a.RHOT0, c, o.T0 + dt * (adt + (double)o.St), o.T0, o.aT);
             if (m <= KE - 1) {
-                const double Cm = CA(sC, cc, m);
-                put_state(a, N3, 1, a.MOMZ_RK, a.MOMZ0, c, ld(a.MOMZ0 + c) + (Cm - ld(a.MOMZ + c)), true);
-                put_flux(a, N3, 0, c, R((double)ld(nd.DZ() + c) + J33G * Cm), true);
-                put_flux(a, N3, 3, c, R((double)__ldcg(stZ + c) + J33G * Cm * CA(sP, cc, m)), true);
+                fold_state<M>(a, ptr, N3, 1, a.MOMZ_RK, a.MOMZ0, c, o.W0 + (Cm - o.W), o.W0, o.aW);
+                fold_flux<M>(a, ptr, N3, 0, c, R((double)o.nDZ + J33G * Cm), o.aM);
+                fold_flux<M>(a, ptr, N3, 3, c, R((double)o.tZ + J33G * Cm * Pm), o.aQ);
             } else {
                 put_state(a, N3, 1, a.MOMZ_RK, a.MOMZ0, c, 0.0, false);
-                put_flux(a, N3, 0, c, R(0.0), true);
-                put_flux(a, N3, 3, c, R(0.0), true);
+                fold_flux<M>(a, ptr, N3, 0, c, R(0.0), o.aM);
+                fold_flux<M>(a, ptr, N3, 3, c, R(0.0), o.aQ);
             }
         }
-        if (lane == 0) {
+        if (m == KS) {
             // rigid-lid and surface values (:753-754) and the zero fluxes at KS-1 (:371, ud3.F90:222)
-            put_state(a, N3, 1, a.MOMZ_RK, a.MOMZ0, col + KS - 2, 0.0, false);
-            put_flux(a, N3, 0, col + KS - 2, R(0.0), false);
-            put_flux(a, N3, 3, col + KS - 2, R(0.0), false);
+            put_state(a, N3, 1, a.MOMZ_RK, a.MOMZ0, c - 1, 0.0, false);
+            put_flux(a, N3, 0, c - 1, R(0.0), false);
+            put_flux(a, N3, 3, c - 1, R(0.0), false);
         }
         // hevi_mflx_z :369-393 also fills the halo column i = IS-1 with the explicit
         // part of the vertical mass flux; the solver never updates it
-        if (i == g.IS && (a.rk_mode == RK_PLAIN || a.rk_mode == RK_FINAL || a.rk_mode == RK_HEUN3)) {
+        if (i == g.IS && item < CCOLS && (a.rk_mode == RK_PLAIN || a.rk_mode == RK_FINAL || a.rk_mode == RK_HEUN3)) {
             const size_t chl = idx3(g, 1, g.IS - 1, j);
             for (int k = KS - 1 + lane; k <= KE; k += 32)
-                a.mflx[chl + k - 1] = (k >= KS && k <= KE - 1) ? ld(nd.DZ() + chl + k - 1) : R(0.0);
+                a.mflx[chl + k - 1] = (k >= KS && k <= KE - 1) ? ld(ptr.nd[0] + chl + k - 1) : R(0.0);
         }
     }
 #undef CA
@@ -742,31 +929,50 @@ __global__ void __launch_bounds__(32 * NWARPS, 1024 / (32 * NWARPS) > 1 ? 2 : 1)
 // =============================================================================
 // host side
 // =============================================================================
+template <int S, int M, typename R>
+cudaError_t launch_pair(const Grid &g, const StageArgsT<R> &a, BatchT<1> B, const StageMaps<R> &h, cudaStream_t st)
+{
+    auto kx = k_hevi_explicit<S, R, M, 1>;
+    cudaError_t e = open_smem(kx, smem_bytes<S>());
+    if (e != cudaSuccess) return e;
+    B.first[1] = ((g.IMAX + TX - 1) / TX) * ((g.JMAX + TY - 1) / TY);
+    kx<<<B.first[1], dim3(32, NCOL), smem_bytes<S>(), st>>>(g, a, B, h.ptr, h.maps);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    auto kc = k_hevi_column<R, M, 1>;
+    // the attribute is set once per device, so it opens the largest size (KA = 260)
+    if ((e = open_smem(kc, column_smem(260))) != cudaSuccess) return e;
+    B.first[1] = ((g.IMAX + CCOLS - 1) / CCOLS) * g.JMAX;
+    kc<<<B.first[1], dim3(32, CWARPS), column_smem(g.KA), st>>>(g, a, B, h.ptr);
+    return cudaGetLastError();
+}
+
 template <int S, typename R>
 cudaError_t launch_s(const Grid &g, StageArgsT<R> a, int raster, cudaStream_t st)
 {
-    StateMaps maps;
+    StageMaps<R> h;
     const double *f[NF] = {a.DENS, a.MOMZ, a.MOMX, a.MOMY, a.RHOT};
     for (int q = 0; q < NF; ++q)
-        if (!encode(&maps.m[q], f[q], g, box_k<S>(), box_w<S>(), box_h<S>())) return cudaErrorNotSupported;
+        if (!encode(&h.maps.m[q], f[q], g, box_k<S>(), box_w<S>(), box_h<S>())) return cudaErrorNotSupported;
+    const size_t N3 = n3(g);
+    for (int q = 0; q < 15; ++q) h.ptr.nd[q] = a.num_diff + q * N3;
+    for (int q = 0; q < 5; ++q) h.ptr.acc[q] = a.acc + q * N3;
+    for (int q = 0; q < 6; ++q) {
+        h.ptr.facc[q] = a.facc + q * N3;
+        h.ptr.flx[q] = (q < 3 ? a.mflx : a.tflx) + (q % 3) * N3;
+    }
+    h.ptr.Sr = a.colscr; h.ptr.St = a.colscr + N3; h.ptr.tZ = a.colscr + 2 * N3; h.ptr.PT = a.colscr + 3 * N3;
     BatchT<1> B{};
     B.n = 1;
     a.raster = raster > 0 ? raster : STAGE_RASTER_DEFAULT;
-    const int ntiles = ((g.IMAX + TX - 1) / TX) * ((g.JMAX + TY - 1) / TY);
     B.first[0] = 0;
-    B.first[1] = ntiles;
-    auto kx = k_hevi_explicit<S, R, 1>;
-    cudaError_t e = open_smem(kx, smem_bytes<S>());
-    if (e != cudaSuccess) return e;
-    kx<<<ntiles, dim3(32, NCOL), smem_bytes<S>(), st>>>(g, a, B, maps);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    auto kc = k_hevi_column<R, 1>;
-    // the attribute is set once per device, so it opens the largest size (KA = 260)
-    if ((e = open_smem(kc, column_smem(260))) != cudaSuccess) return e;
-    const int ncb = ((g.IMAX + CCOLS - 1) / CCOLS) * g.JMAX;
-    B.first[1] = ncb;
-    kc<<<ncb, dim3(32, CWARPS), column_smem(g.KA), st>>>(g, a, B);
-    return cudaGetLastError();
+    switch (a.rk_mode) {
+    case RK_PLAIN: return launch_pair<S, RK_PLAIN>(g, a, B, h, st);
+    case RK_STAGE1: return launch_pair<S, RK_STAGE1>(g, a, B, h, st);
+    case RK_STAGE2:
+    case RK_STAGE3: return launch_pair<S, RK_STAGE2>(g, a, B, h, st);
+    case RK_FINAL: return launch_pair<S, RK_FINAL>(g, a, B, h, st);
+    default: return launch_pair<S, FOLD_ANY>(g, a, B, h, st);
+    }
 }
 
 template <typename R>
