@@ -38,6 +38,9 @@ CPP_SOURCES = ["grid_coef.cpp"]
 # these sources, with -DHEVI_FLOAT_TU and FMA contraction on: their results are
 # held to a tolerance against the FP64 path, not bit for bit, so a*b+c may fuse.
 FLOAT_SOURCES = ["hevi_stage.cu", "hevi_tma.cu", "numfilter.cu", "tracer.cu", "persist.cu"]
+# The tiled stage's instantiations without tensor maps compile from the same
+# source with -DHEVI_COPY_TU, so that the two long builds run side by side.
+COPY_SOURCE = "hevi_tma.cu"
 HEADERS = ["hevi_common.cuh", "hevi_stage.cuh", "hevi_kernels.cuh", "hevi_epilogue.cuh", "adjoint.cuh",
            "numfilter_body.cuh", "fill_body.cuh", "hevi_stage_body.cuh", "rn_div.cuh", "tma_util.cuh", "grid_coef.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -86,6 +89,10 @@ def build_cuda(force: bool = False, verbose: bool = False) -> Path:
     for src in FLOAT_SOURCES:
         obj = objdir / (Path(src).stem + "_f32.o")
         cmds.append([nvcc, *f32, *ARCH, "-c", str(CSRC / src), "-o", str(obj)] + (["-Xptxas", "-v"] if verbose else []))
+        objs.append(str(obj))
+    for flags, obj in ((common, objdir / "hevi_copy.o"), (f32, objdir / "hevi_copy_f32.o")):
+        cmds.append([nvcc, *flags, "-DHEVI_COPY_TU", *ARCH, "-c", str(CSRC / COPY_SOURCE), "-o", str(obj)]
+                    + (["-Xptxas", "-v"] if verbose else []))
         objs.append(str(obj))
     # the translation units compile independently; the kernel templates make
     # some of them long, so they run side by side

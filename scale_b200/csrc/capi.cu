@@ -57,8 +57,7 @@ struct Ctx {
     std::vector<double> nd_key;
     NdCoef ndc{};
     // scratch
-    double *rk[2] = {nullptr, nullptr}; // 5*N3 each
-    double *acc = nullptr;          // 5*N3
+    double *rk[3] = {nullptr, nullptr, nullptr}; // stage buffers, 5*N3 each
     double *facc = nullptr;         // 6*N3
     double *colscr = nullptr;       // 4*N3: Sr, St, tZ (fused and tiled stage), PT (tiled stage)
     double *colC = nullptr;         // 2*N3: the column problem's right-hand side, then f, and e (tiled stage)
@@ -201,7 +200,7 @@ int falloc(float **p, size_t n)
 
 void free_all()
 {
-    double *bufs[] = {C.eng_part, C.phi, C.ndw, C.colscr, C.colC, C.d_tab, C.d_nd, C.rk[0], C.rk[1], C.acc, C.facc, C.tr, C.lg, C.sum_part, C.sum_out,
+    double *bufs[] = {C.eng_part, C.phi, C.ndw, C.colscr, C.colC, C.d_tab, C.d_nd, C.rk[0], C.rk[1], C.rk[2], C.facc, C.tr, C.lg, C.sum_part, C.sum_out,
                       C.tw_buf};
     for (double *b : bufs) if (b) cudaFree(b);
     for (auto &kv : C.stage) cudaFree(kv.second.first);
@@ -516,7 +515,7 @@ StageArgsT<F> stage_args(const StageInT<F> &in, double *const out[5], F *mflx, F
     a.DPRES0 = in.DPRES0; a.RT2P = in.RT2P; a.CORIOLI = in.CORIOLI; a.num_diff = in.num_diff;
     a.wdamp = C.d_wdamp; a.DDIV = in.DDIV; a.REF_dens = in.REF_dens; a.REF_rhot = in.REF_rhot;
     a.divdmp_coef = in.divdmp; a.J33G = in.J33G; a.dtrk = dtrk;
-    a.rk_mode = mode; a.acc = mode == RK_HEUN3 ? C.rk[0] : C.acc; a.facc = facc_buf<F>(); a.status = C.status;
+    a.rk_mode = mode; a.rk1 = C.rk[0]; a.rk2 = C.rk[1]; a.rk3 = C.rk[2]; a.facc = facc_buf<F>(); a.status = C.status;
     a.colscr = colscr_buf<F>();
     a.colC = C.colC;
     return a;
@@ -545,6 +544,7 @@ int autotune_stage(const StageInT<F> &in, double dtrk)
     int rc = SCALE_HEVI_OK;
     constexpr int FORMS[4] = {0, STAGE_TILE_XS[0], STAGE_TILE_XS[1], STAGE_TILE_XS[2]};
     for (int tx : FORMS) {
+        if (tx == 0 && C.members.size() > 1) continue; // an ensemble's shapes are those of the fused kernel
         for (int r : RASTERS) {
             const StageShape sh{tx, r};
             int nl = 1;
@@ -644,7 +644,7 @@ int run_rk4(double *X[5], F *mflx, F *tflx, const StageInT<F> &base, double dt)
         in.DENS = src[0]; in.MOMZ = src[1]; in.MOMX = src[2]; in.MOMY = src[3]; in.RHOT = src[4];
         double *out[5];
         if (s < 3) {
-            double *b = C.rk[s % 2];
+            double *b = C.rk[s];
             for (int v = 0; v < 5; ++v) out[v] = b + (size_t)v * C.N3;
         } else {
             for (int v = 0; v < 5; ++v) out[v] = X[v];
@@ -904,7 +904,7 @@ int scale_hevi_ensemble_setup(int n, const scale_hevi_index *idx, const char *fl
     if ((rc = dalloc(&C.d_tab, 7 * (size_t)ZT + 4 * (size_t)XT + 4 * (size_t)YT)) ||
         (rc = dalloc(&C.d_nd, 18 * (size_t)ZT + 18 * (size_t)XT + 18 * (size_t)YT)) ||
         (rc = dalloc(&C.rk[0], 5 * N3)) || (rc = dalloc(&C.rk[1], 5 * N3)) ||
-        (rc = dalloc(&C.acc, 5 * N3)) || (rc = dalloc(&C.facc, 6 * N3)) ||
+        (rc = dalloc(&C.rk[2], 5 * N3)) || (rc = dalloc(&C.facc, 6 * N3)) ||
         (rc = dalloc(&C.colscr, 4 * N3)) || (rc = dalloc(&C.colC, 2 * N3)) ||
         (rc = dalloc(&C.sum_part, (size_t)x.IMAX * x.JMAX)) || (rc = dalloc(&C.sum_out, 1))) {
         free_all();
@@ -1326,7 +1326,7 @@ int short_step_persistent(double *X[5], R *mflx, R *tflx, R *num_diff, const R *
     for (int s = 0; s < 4; ++s) {
         in.DENS = src[0]; in.MOMZ = src[1]; in.MOMX = src[2]; in.MOMY = src[3]; in.RHOT = src[4];
         double *out[5];
-        for (int v = 0; v < 5; ++v) out[v] = s < 3 ? C.rk[s % 2] + (size_t)v * C.N3 : X[v];
+        for (int v = 0; v < 5; ++v) out[v] = s < 3 ? C.rk[s] + (size_t)v * C.N3 : X[v];
         p.st[s] = stage_args(in, out, mflx, tflx, dts[s], RK_STAGE1 + s);
         if (s < 3)
             for (int v = 0; v < 5; ++v) { p.rk[s][v] = out[v]; src[v] = out[v]; }

@@ -31,21 +31,23 @@ template <typename F>
 __device__ __forceinline__ void put_state(const StageArgsT<F> &a, size_t N3, int v, double *out, const double *x0,
                                           size_t c, double val, bool combine)
 {
-    double *acc = a.acc + (size_t)v * N3 + c;
+    const size_t q = (size_t)v * N3 + c;
     switch (a.rk_mode) {
     case RK_PLAIN: sts(out + c, val); flag_nonfinite(a.status, val); break;
-    case RK_STAGE1: sts(out + c, val); if (combine) sts(acc, val * 2.0); break;
-    case RK_STAGE2: sts(out + c, val); if (combine) sts(acc, lds(acc) + val * 4.0); break;
-    case RK_STAGE3: sts(out + c, val); if (combine) sts(acc, lds(acc) + val * 2.0); break;
+    case RK_STAGE1:
+    case RK_STAGE2:
+    case RK_STAGE3:
     case RK_HEUN1: sts(out + c, val); break;
     case RK_HEUN3: {
-        double r = combine ? ((lds(acc) * 3.0 + val * 3.0) - lds(x0 + c) * 2.0) / 4.0 : val;
+        double r = combine ? ((lds(a.rk1 + q) * 3.0 + val * 3.0) - lds(x0 + c) * 2.0) / 4.0 : val;
         sts(out + c, r);
         flag_nonfinite(a.status, r);
         break;
     }
     default: {
-        double r = combine ? ((lds(acc) + val) - lds(x0 + c) * 3.0) / 6.0 : val;
+        double r = combine ? ((((lds(a.rk1 + q) * 2.0 + lds(a.rk2 + q) * 4.0) + lds(a.rk3 + q) * 2.0) + val)
+                              - lds(x0 + c) * 3.0) / 6.0
+                           : val;
         sts(out + c, r);
         flag_nonfinite(a.status, r);
     }

@@ -157,7 +157,7 @@ void divergence_terrain(const Grid &g, double *DDIV, const double *MOMZ, const d
 
 // ---- HEVI stage (hevi_stage.cu) ----
 // Form and launch shape of the stage. tile_x = 0: the tiled stage (hevi_tma.cu:
-// 4 x 4 column tiles staged by bulk tensor copies) where it applies, else the
+// 4 x 4 column tiles staged in shared memory) where it applies, else the
 // fused kernel with its default tile;
 // tile_x = 16, 8 or 4: the fused kernel k_hevi_stage with a tile of tile_x x
 // (16/tile_x) columns. raster: rows of tiles per raster group; 0 selects the default.
@@ -172,11 +172,15 @@ constexpr int STAGE_RASTER_DEFAULT = 16;
 template <typename R>
 cudaError_t launch_hevi_stage(const Grid &g, const Members &mem, const StageArgsT<R> &a, int scheme, StageShape shape,
                               cudaStream_t st, int *launches = nullptr, bool *tiled = nullptr);
-// the tiled stage alone; cudaErrorNotSupported where it does not apply (an
-// ensemble, odd KA, a field off a 16-byte boundary, no tiled column scratch)
+// the tiled stage alone; cudaErrorNotSupported where it does not apply (a mixed-precision
+// ensemble, no tiled column scratch)
 template <typename R>
 cudaError_t launch_hevi_stage_tiled(const Grid &g, const Members &mem, const StageArgsT<R> &a, int scheme, int raster,
                                     cudaStream_t st);
+// its form that stages without tensor maps (any KA and alignment, any members)
+template <typename R>
+cudaError_t launch_hevi_stage_copied(const Grid &g, const Members &mem, const StageArgsT<R> &a, int scheme, int raster,
+                                     cudaStream_t st);
 // one HEVE stage (FP64), same arguments; the RK4 combine modes apply as for HEVI
 cudaError_t launch_heve_stage(const Grid &g, const Members &mem, const StageArgsT<double> &a, int scheme,
                               cudaStream_t st);

@@ -9,18 +9,21 @@ namespace hevi {
 // write their outputs to RK buffers and the combine (:562-650) forms
 //   X  = (RK1*2 + RK2*4 + RK3*2 + X4 - X0*3) / 6      (state, interior)
 //   F  = (F1 + F2*2 + F3*2 + F4) / 6                    (mflx_hi/tflx_hi, interior)
-// Accumulating the same sums left to right in the stage epilogues gives the
-// identical IEEE results without storing RK1..RK3 fluxes or a combine pass.
+// The last stage's epilogue forms X from the three stage buffers, which the
+// stages write anyway (accumulating the sum as the stages go would read and
+// write five more fields in each of them); the flux sums, whose stage values
+// nothing else needs, accumulate left to right in the epilogues. Both give the
+// identical IEEE results without a combine pass.
 enum RkMode : int {
     RK_PLAIN = 0,  // one ATMOS_DYN_Tstep_short call: outputs only
-    RK_STAGE1 = 1, // acc = X*2, facc = F
-    RK_STAGE2 = 2, // acc += X*4, facc += F*2
-    RK_STAGE3 = 3, // acc += X*2, facc += F*2
-    RK_FINAL = 4,  // X = ((acc + X) - X0*3)/6, F = (facc + F)/6 over the interior
+    RK_STAGE1 = 1, // facc = F
+    RK_STAGE2 = 2, // facc += F*2
+    RK_STAGE3 = 3, // facc += F*2
+    RK_FINAL = 4,  // X = (RK1*2 + RK2*4 + RK3*2 + X - X0*3)/6, F = (facc + F)/6 over the interior
     // Heun's RK3 (scale_atmos_dyn_tinteg_short_rk3.F90:188-576): stage 1 writes
     // RK1 to its buffer and F1 to facc; stage 2 is RK_PLAIN; stage 3 forms
     //   X = ((RK1*3 + X3*3) - X0*2)/4, F = (F1 + F3*3)/4 over the interior
-    // with acc pointing at the stage-1 buffer.
+    // with rk1 pointing at the stage-1 buffer.
     RK_HEUN1 = 5,
     RK_HEUN3 = 6,
 };
@@ -53,7 +56,7 @@ struct StageArgsT {
     double divdmp_coef, J33G, dtrk;
     // RK accumulation
     int rk_mode;
-    double *acc; // 5*N3: DENS, MOMZ, MOMX, MOMY, RHOT
+    const double *rk1, *rk2, *rk3; // stage buffers, 5*N3 each: DENS, MOMZ, MOMX, MOMY, RHOT
     F *facc;     // 6*N3: mflx Z,X,Y then tflx Z,X,Y
     unsigned *status;
     F *colscr; // Sr, St, tZ (3*N3, the fused kernel) and PT (4*N3, the tiled kernels)

@@ -217,7 +217,7 @@ extern "C" int ATMOS_DYN_Tstep_short_fvm_hevi_b200_noalloc(const scale_hevi_inde
     a.DPRES0 = DPRES0; a.RT2P = RT2P; a.CORIOLI = CORIOLI; a.num_diff = num_diff;
     a.wdamp = z + 6 * KA; a.DDIV = DDIV; a.REF_dens = REF_dens; a.REF_rhot = REF_rhot;
     a.divdmp_coef = *divdmp_coef; a.J33G = *J33G; a.dtrk = *dtrk;
-    a.rk_mode = RK_PLAIN; a.acc = nullptr; a.facc = nullptr; a.status = status;
+    a.rk_mode = RK_PLAIN; a.rk1 = a.rk2 = a.rk3 = nullptr; a.facc = nullptr; a.status = status;
     a.colscr = HEVI_COL_SCRATCH ? colscr : nullptr;
 
     NA_CU(launch_hevi_stage(g, Members{}, a, scheme, StageShape{}, st));
