@@ -31,13 +31,13 @@ LIB = LIBDIR / "libscale_hevi.so"
 ORACLE_DIR = ROOT / "oracle"
 ORACLE_LIB = ORACLE_DIR / "build" / "liboracle.so"
 
-CU_SOURCES = ["capi.cu", "hevi_stage.cu", "hevi_tma.cu", "numfilter.cu", "tracer.cu", "misc.cu", "noalloc.cu",
+CU_SOURCES = ["capi.cu", "hevi_stage.cu", "hevi_tma.cu", "numfilter.cu", "numfilter_tiled.cu", "tracer.cu", "misc.cu", "noalloc.cu",
               "persist.cu", "adjoint.cu"]
 CPP_SOURCES = ["grid_coef.cpp"]
 # The FP32 instantiations of the mixed-precision path compile a second time from
 # these sources, with -DHEVI_FLOAT_TU and FMA contraction on: their results are
 # held to a tolerance against the FP64 path, not bit for bit, so a*b+c may fuse.
-FLOAT_SOURCES = ["hevi_stage.cu", "hevi_tma.cu", "numfilter.cu", "tracer.cu", "persist.cu"]
+FLOAT_SOURCES = ["hevi_stage.cu", "hevi_tma.cu", "numfilter.cu", "numfilter_tiled.cu", "tracer.cu", "persist.cu"]
 # The tiled stage's instantiations without tensor maps compile from the same
 # source with -DHEVI_COPY_TU, so that the two long builds run side by side.
 COPY_SOURCE = "hevi_tma.cu"

@@ -37,7 +37,6 @@
 // Flat terrain.
 #include "hevi_epilogue.cuh"
 #include "hevi_kernels.cuh"
-#include "numfilter_body.cuh"
 #include "rn_div.cuh"
 #include "tma_util.cuh"
 
@@ -65,17 +64,6 @@ template <int S> constexpr size_t smem_bytes()
 {
     return (size_t)NF * plane<S>() * sizeof(double) + (size_t)((DP_COLS + NCOL + NLT) * NDP + NCOL * NCARRY) * sizeof(double) + 16;
 }
-
-// asynchronous copy of one value into shared memory, from this thread's view
-// complete after copy_wait
-template <typename T>
-__device__ __forceinline__ void copy_async(T *dst, const T *src)
-{
-    static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async sizes");
-    if constexpr (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 struct StateMaps {
     CUtensorMap m[NF]; // DENS, MOMZ, MOMX, MOMY, RHOT as (KA, IA, JA) FP64 tensors
@@ -161,13 +149,6 @@ __device__ __forceinline__ void rim_flux(const StageArgsT<R> &a, const StagePtrs
     if constexpr (M == RK_PLAIN || M == RK_FINAL) sts(p.flx[f] + c, val);
     else if constexpr (M == FOLD_ANY) put_flux(a, N3, f, (size_t)c, val, false);
 }
-
-// How the state fields come into shared memory: LD_TMA, bulk tensor copies; LD_COPY,
-// cp.async of single values by every thread, for an ensemble (whose members would
-// each need tensor maps) and for odd KA or unaligned fields, which admit none.
-// LD_COPY costs 24 copies per thread and chunk and one barrier more: 5% on a domain
-// that admits both.
-enum Loader : int { LD_TMA = 0, LD_COPY = 1 };
 
 template <int S, typename R, int M, int LD, int NM>
 __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
@@ -900,117 +881,6 @@ __global__ void __launch_bounds__(32 * CWARPS, 4)
 #undef CA
 }
 
-#ifndef HEVI_COPY_TU
-// =============================================================================
-// k_numfilter_tiled: the 15 num_diff components (ND_ORDER = 1) of a 4 x 4 tile
-// of columns from shared memory
-// =============================================================================
-// One warp per column, lanes along k, chunks of 32 levels as in
-// k_hevi_explicit. Per chunk one thread copies the five filtered quantities
-// (phi, written by k_phi) and DENS over the tile, a lateral halo of 2 and the
-// levels L0-2..L0+33 into shared memory (six bulk tensor copies completing on
-// an mbarrier, bounded wait); numfilter_cell then forms every component from
-// there, with the arithmetic of k_numfilter, so the two give identical bits.
-// The vertical halo levels of each column follow with global loads.
-#ifndef HEVI_ND_TX
-#define HEVI_ND_TX 4
-#define HEVI_ND_TY 4
-#endif
-constexpr int NTX = HEVI_ND_TX, NTY = HEVI_ND_TY, NWARPS = NTX * NTY; // tile columns; one warp each
-constexpr int NKLO = 2;                        // box levels below the chunk's first
-constexpr int NBK = KC + 4;                    // box levels: L0-2 .. L0+33
-constexpr int NBW = NTX + 4, NBH = NTY + 4;    // lateral halo of 2
-constexpr int NPL = NBK * NBW * NBH;           // one staged field
-template <typename R> constexpr size_t nd_smem_bytes() { return (size_t)NPL * (5 * sizeof(R) + sizeof(double)) + 16; }
-
-struct NdMaps {
-    CUtensorMap m[6]; // phi q = 0..4 (type R), DENS (FP64), as (KA, IA, JA) tensors
-};
-
-// the staged filtered quantities; box element 0 is level k0, column i0, row j0
-template <typename R>
-struct PhiS {
-    using type = R;
-    const R *base;
-    int k0, i0, j0;
-    __device__ R operator()(int q, int k, int i, int j) const
-    {
-        return base[q * NPL + ((j - j0) * NBW + (i - i0)) * NBK + (k - k0)];
-    }
-};
-// the staged density around a cell
-struct DensS {
-    const double *p;
-    __device__ double operator()(int dk, int di, int dj) const { return p[dk + di * NBK + dj * NBK * NBW]; }
-};
-
-template <typename R>
-__global__ void __launch_bounds__(32 * NWARPS, 1024 / (32 * NWARPS) > 1 ? 2 : 1)
-    k_numfilter_tiled(const Grid g, const NdCoef c, const NdArgsT<R> a, unsigned *status,
-                      const __grid_constant__ NdMaps maps)
-{
-    extern __shared__ __align__(1024) double sm[];
-    R *sphi = reinterpret_cast<R *>(sm); // 5 fields, [j][i][k] each
-    double *sdn = reinterpret_cast<double *>(reinterpret_cast<char *>(sm) + (size_t)5 * NPL * sizeof(R));
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sdn + NPL);
-    __shared__ int s_ok;
-    const int lane = threadIdx.x, w = threadIdx.y, tid = w * 32 + lane;
-    const int tx = w % NTX, ty = w / NTX;
-    const int nti = (g.IMAX + NTX - 1) / NTX;
-    const int i0 = g.IS + ((int)blockIdx.x % nti) * NTX, j0 = g.JS + ((int)blockIdx.x / nti) * NTY;
-    const int i = i0 + tx, j = j0 + ty;
-    const bool col_ok = i <= g.IE && j <= g.JE;
-    const size_t N3 = n3(g);
-    const int KS = g.KS, KE = g.KE;
-    const int NC = (g.KMAX + KC - 1) / KC;
-    constexpr unsigned BYTES = (unsigned)(NPL * (5 * sizeof(R) + sizeof(double)));
-
-    auto issue = [&](int ch) {
-        // box origin (0-based): level L0-2 = 32*ch (KS = 3), column i0-2, row j0-2
-        const int x = KC * ch + (KS - 1) - NKLO, y = i0 - 2 - 1, z = j0 - 2 - 1;
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(bar, BYTES);
-        for (int q = 0; q < 5; ++q) tma_load_3d(sphi + (size_t)q * NPL, &maps.m[q], x, y, z, bar);
-        tma_load_3d(sdn, &maps.m[5], x, y, z, bar);
-    };
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        issue(0);
-    }
-    __syncthreads();
-
-    const R ncx = col_ok ? R(ld(c.cdx + i - 1)) : R(0.0), nfx = col_ok ? R(ld(c.fdx + i - 1)) : R(0.0);
-    const R ncy = col_ok ? R(ld(c.cdy + j - 1)) : R(0.0), nfy = col_ok ? R(ld(c.fdy + j - 1)) : R(0.0);
-    const R sfc = R(c.sfc);
-    for (int ch = 0; ch < NC; ++ch) {
-        if (tid == 0) {
-            const bool ok = mbar_wait(bar, ch & 1);
-            // on a timeout, wait once more (bounded) for the copies still in flight
-            if (!ok) (void)mbar_wait(bar, ch & 1);
-            s_ok = ok ? 1 : 0;
-        }
-        __syncthreads();
-        if (!s_ok) {
-            if (tid == 0) atomicOr(status, ST_TMA_TIMEOUT);
-            return; // block-uniform
-        }
-        (void)mbar_try(bar, ch & 1); // completed phase: makes the copied data visible to this thread
-        const int L0 = KS + KC * ch, k = L0 + lane;
-        if (col_ok && k <= KE) {
-            const PhiS<R> phi{sphi, L0 - NKLO, i0 - 2, j0 - 2};
-            const DensS dn{sdn + ((ty + 2) * NBW + (tx + 2)) * NBK + (k - (L0 - NKLO))};
-            numfilter_cell<false>(g, c, phi, dn, nullptr, a.num_diff, N3, idx3(g, k, i, j), k, i, j, ncx, nfx, ncy,
-                                  nfy, sfc);
-        }
-        __syncthreads(); // every read of the staged box is done
-        if (tid == 0 && ch + 1 < NC) issue(ch + 1);
-    }
-    if (col_ok) numfilter_halo_levels<false>(g, c, Phi<R>{g, a}, nullptr, a.num_diff, N3, a.DENS, i, j, lane);
-}
-
-#endif // HEVI_COPY_TU
-
 // =============================================================================
 // host side
 // =============================================================================
@@ -1092,44 +962,9 @@ cudaError_t launch_scheme(const Grid &g, const Members &mem, const StageArgsT<R>
     }
 }
 
-#ifndef HEVI_COPY_TU
-template <typename R>
-cudaError_t launch_numfilter_s(const Grid &g, const NdCoef &c, const NdArgsT<R> &a, unsigned *status, cudaStream_t st)
-{
-    NdMaps maps;
-    for (int q = 0; q < 5; ++q)
-        if (!encode(&maps.m[q], a.phi + (size_t)q * n3(g), g, NBK, NBW, NBH)) return cudaErrorNotSupported;
-    if (!encode(&maps.m[5], a.DENS, g, NBK, NBW, NBH)) return cudaErrorNotSupported;
-    auto k = k_numfilter_tiled<R>;
-    cudaError_t e = open_smem(k, nd_smem_bytes<R>());
-    if (e != cudaSuccess) return e;
-    const int ntiles = ((g.IMAX + NTX - 1) / NTX) * ((g.JMAX + NTY - 1) / NTY);
-    k<<<ntiles, dim3(32, NWARPS), nd_smem_bytes<R>(), st>>>(g, c, a, status, maps);
-    return cudaGetLastError();
-}
-
-#endif // HEVI_COPY_TU
 }  // namespace tma
 
 #ifndef HEVI_COPY_TU
-// The numerical filter's components from staged tiles where they apply: one
-// domain of KHALO = 2 whose filtered quantities and density admit tensor maps
-// (16-byte aligned bases and strides). cudaErrorNotSupported otherwise.
-template <typename R>
-cudaError_t launch_numfilter_tiled(const Grid &g, const Members &mem, const NdCoef &c, const NdArgsT<R> &a,
-                                   unsigned *status, cudaStream_t st)
-{
-    if (mem.n > 1 || g.KS != 3 || c.order != 1 || !status) return cudaErrorNotSupported;
-    return tma::launch_numfilter_s<R>(g, c, a, status, st);
-}
-#ifndef HEVI_FLOAT_TU
-template cudaError_t launch_numfilter_tiled<double>(const Grid &, const Members &, const NdCoef &,
-                                                    const NdArgsT<double> &, unsigned *, cudaStream_t);
-#else
-template cudaError_t launch_numfilter_tiled<float>(const Grid &, const Members &, const NdCoef &,
-                                                   const NdArgsT<float> &, unsigned *, cudaStream_t);
-#endif
-
 // The tiled stage where it applies: one domain or, in FP64, an ensemble, KA <= 260 and
 // the column scratch of the tiled kernels present. cudaErrorNotSupported otherwise
 // (the caller then runs the fused kernel). One domain of even KA whose fields lie on

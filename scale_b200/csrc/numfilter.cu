@@ -141,7 +141,7 @@ cudaError_t launch_numfilter(const Grid &g, const Members &mem, const NdCoef &c,
         return cudaSuccess;
     });
     if (status) {
-        // one domain: the components from staged tiles where the tensor maps apply
+        // the components from staged tiles
         const cudaError_t e = launch_numfilter_tiled(g, mem, c, a, status, st);
         if (e != cudaErrorNotSupported) return e;
     }

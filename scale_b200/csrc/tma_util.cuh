@@ -1,4 +1,5 @@
-// Tensor-memory-accelerator plumbing shared by the tiled kernels: mbarrier
+// Copies into shared memory shared by the tiled kernels: cp.async, and the tensor
+// memory accelerator's plumbing: mbarrier
 // operations with bounded waits, the 3-D bulk tensor load into shared memory,
 // the tensor-map encoder (through the driver entry point, no link against
 // libcuda) and the one-time opening of a kernel's dynamic shared memory.
@@ -59,6 +60,24 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 // a following bulk copy into it
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+
+// asynchronous copy of one value into shared memory, from this thread's view
+// complete after copy_wait
+template <typename T>
+__device__ __forceinline__ void copy_async(T *dst, const T *src)
+{
+    static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async sizes");
+    if constexpr (sizeof(T) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// How a kernel's boxes come into shared memory: LD_TMA, bulk tensor copies; LD_COPY,
+// cp.async of single values by every thread, for an ensemble (whose members would
+// each need tensor maps) and for arrays that admit none (strides or bases off 16
+// bytes). In the stage LD_COPY costs 24 copies per thread and chunk and one barrier
+// more: about 5% on a domain that admits both.
+enum Loader : int { LD_TMA = 0, LD_COPY = 1 };
 
 static inline PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
 {
