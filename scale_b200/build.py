@@ -31,8 +31,8 @@ LIB = LIBDIR / "libscale_hevi.so"
 ORACLE_DIR = ROOT / "oracle"
 ORACLE_LIB = ORACLE_DIR / "build" / "liboracle.so"
 
-CU_SOURCES = ["capi.cu", "hevi_stage.cu", "hevi_tma.cu", "numfilter.cu", "numfilter_tiled.cu", "tracer.cu", "misc.cu", "noalloc.cu",
-              "persist.cu", "adjoint.cu"]
+CU_SOURCES = ["capi.cu", "hevi_stage.cu", "hevi_tma.cu", "hevi_terrain.cu", "numfilter.cu", "numfilter_tiled.cu",
+              "tracer.cu", "misc.cu", "noalloc.cu", "persist.cu", "adjoint.cu"]
 CPP_SOURCES = ["grid_coef.cpp"]
 # The FP32 instantiations of the mixed-precision path compile a second time from
 # these sources, with -DHEVI_FLOAT_TU and FMA contraction on: their results are

@@ -12,7 +12,7 @@
 // before any launch): the metric factors then multiply or divide by exactly 1
 // and the J13/J23 flux terms are exact zeros, so dropping them leaves every
 // non-zero value unchanged. Other metrics go to the general-metric stage
-// (terrain_stage in hevi_stage.cu), which keeps every metric term.
+// (hevi_terrain.cu), which keeps every metric term.
 #pragma once
 #include <cstddef>
 #include <cstdint>

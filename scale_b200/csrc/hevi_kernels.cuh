@@ -57,7 +57,7 @@ cudaError_t with_batch(const Grid &g, const Members &mem, NB nblocks_of, L launc
 struct Block2 { int x, y; };
 __device__ __forceinline__ Block2 split_block(int b, int gx) { return {b % gx, b / gx}; }
 
-// ---- the HEVI stage with terrain-following metrics (hevi_stage.cu) ----
+// ---- the HEVI stage with terrain-following metrics (hevi_terrain.cu; HEVE: hevi_stage.cu) ----
 // GSQRT, J13G, J23G (KA,IA,JA,7), MAPF (IA,JA,2,4), PHI (KA,IA,JA): device arrays
 struct Metrics {
     const double *GSQRT, *J13G, *J23G, *MAPF, *PHI;
@@ -69,7 +69,7 @@ struct TerrainWork {
     double *A, *PT, *F1, *F2, *F3, *C, *e, *f;
 };
 constexpr int TERRAIN_WORK_FIELDS = 24;
-constexpr int TERRAIN_STAGE_LAUNCHES = 26; // kernels of one general-metric stage
+constexpr int TERRAIN_STAGE_LAUNCHES = 6; // kernels of one general-metric stage
 constexpr int TERRAIN_HEVE_LAUNCHES = 23;  // kernels of one general-metric HEVE stage
 cudaError_t launch_terrain_heve_stage(const Grid &g, const StageArgsT<double> &a, const Metrics &M,
                                       const TerrainWork &W, int scheme, cudaStream_t st);
