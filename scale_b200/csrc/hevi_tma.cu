@@ -81,6 +81,18 @@ __device__ __forceinline__ R zface_in(R vel, int m, const V &v)
     else return ip4<S>(vel, v(m - 1), v(m), v(m + 1), v(m + 2));
 }
 
+// -(dq r) - (A a + B b), a momentum's vertical and horizontal flux divergence. FP64
+// code never fuses; FP32 code fuses A a into the horizontal sum and nothing else, whatever
+// else the compiler sees around it (the fused stage kernel's rounding)
+__device__ __forceinline__ double advection(double dq, double r, double A, double a, double B, double b)
+{
+    return -dq * r + -(A * a + B * b);
+}
+__device__ __forceinline__ float advection(float dq, float r, float A, float a, float B, float b)
+{
+    return __fadd_rn(__fmul_rn(-dq, r), -__fmaf_rn(A, a, __fmul_rn(B, b)));
+}
+
 // keeps the compiler from carrying values of the fast path into the rare exact one
 __device__ __forceinline__ void cold() { asm volatile("" ::: "memory"); }
 
@@ -459,7 +471,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                 const int k = L - 1;
                 const bool vc = col_ok && (!EDGE || (k >= KS && k <= KE - 1));
                 const double *cMZ = sMZ - 1, *cDN = sDN - 1, *cMX = sMX - 1, *cMY = sMY - 1; // level k
-                R q_k, adv_w = R(0.0);
+                R q_k, dX = R(0.0), dY = R(0.0);
                 auto fluxes = [&](auto fast) {
                     constexpr bool FAST = decltype(fast)::value;
                     rn::Guard<R> gd;
@@ -491,7 +503,8 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                         const R qXw = vXw * ip6<S>(vXw, W_m3, W_m2, W_m1, W_00, W_p1, W_p2) + nXw;
                         const R qYn = vYn * ip6<S>(vYn, V_m2, V_m1, W_00, V_p1, V_p2, V_p3) + nYn;
                         const R qYs = vYs * ip6<S>(vYs, V_m3, V_m2, V_m1, W_00, V_p1, V_p2) + nYs;
-                        adv_w = -((qXe - qXw) * rcdx + (qYn - qYs) * rcdy);
+                        dX = qXe - qXw;
+                        dY = qYn - qYs;
                     }
                     return gd.bad();
                 };
@@ -501,10 +514,10 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                 }
                 const R q_km = below(q_k, C_QW);
                 if (vc) {
-                    const R advcv = -(q_k - q_km) * R(rfdz_k);
+                    const R adv = advection(q_k - q_km, R(rfdz_k), dX, rcdx, dY, rcdy);
                     const R wdmp = -R(wd_k) * R(W0);
                     const R div = use_div ? ddc * (ld(a.DDIV + ck + 1) - ld(a.DDIV + ck)) * R(fdz_k) : R(0.0);
-                    const R Sw = (advcv + adv_w) + wdmp + div + tW;
+                    const R Sw = adv + wdmp + div + tW;
                     const double rfdz = rfdz_k;
                     const double pg = -(dpc[1] + rtc[1] * dt * (double)St - dpc[0] - rtc[0] * dt * (double)St_k) * rfdz * J33G
                                       - GRAV * (f1_k * (cDN[1] - rd1 + (double)Sr * dt)
@@ -524,7 +537,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                 const R cor_u = R(0.125) * (R(ld(a.CORIOLI + g.c2 + (i) + (size_t)g.IA * (j - 1)))
                                             + R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j - 1))));
                 const double dpe = sdp[dpE]; // DPRES at (i+1, j)
-                R q_k, advch;
+                R q_k, dX, dY;
                 auto fluxes = [&](auto fast) {
                     constexpr bool FAST = decltype(fast)::value;
                     rn::Guard<R> gd;
@@ -554,7 +567,8 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                                               R(sMX[2 * KY]), W6 ? R(sMX[3 * KY]) : R(0.0)) + nYn;
                     const R qYs = vS * ip6<S>(vS, W6 ? R(sMX[-3 * KY]) : R(0.0), R(sMX[-2 * KY]), R(sMX[-KY]), U_00,
                                               R(sMX[KY]), W6 ? R(sMX[2 * KY]) : R(0.0)) + nYs;
-                    advch = -((qXe - qXw) * R(rfdx) + (qYn - qYs) * rcdy);
+                    dX = qXe - qXw;
+                    dY = qYn - qYs;
                     return gd.bad() && vb;
                 };
                 if (fluxes(std::true_type{})) {
@@ -563,11 +577,11 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                 }
                 const R q_km = below(q_k, C_QU);
                 if (vb && i <= g.IEH) {
-                    const R advcv = -(q_k - q_km) * R(rcdz_L);
+                    const R adv = advection(q_k - q_km, R(rcdz_L), dX, R(rfdx), dY, rcdy);
                     const double pg = (dpe - dpc[1]) * rfdx;
                     const R cf = cor_u * (R(sMY[KX]) + R(sMY[0]) + R(sMY[KX - KY]) + R(sMY[-KY]));
                     const R div = !use_div ? R(0.0) : ddc * (ld(a.DDIV + c + sI) - ld(a.DDIV + c)) * fdx;
-                    const double val = U0 + dt * (((((double)(advcv + advch)) - pg) + (double)cf) + (double)div + (double)tU);
+                    const double val = U0 + dt * (((((double)adv) - pg) + (double)cf) + (double)div + (double)tU);
                     fold_state<M>(a, ptr, N3, 2, a.MOMX_RK, a.MOMX0, c, val, U0, aU);
                 }
             }
@@ -581,7 +595,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                 const R cor_v = R(-0.125) * (R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j)))
                                              + R(ld(a.CORIOLI + g.c2 + (i - 1) + (size_t)g.IA * (j - 1))));
                 const double dpn = sdp[dpN]; // DPRES at (i, j+1)
-                R q_k, advch;
+                R q_k, dX, dY;
                 auto fluxes = [&](auto fast) {
                     constexpr bool FAST = decltype(fast)::value;
                     rn::Guard<R> gd;
@@ -611,7 +625,8 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                     const R Y_m3 = W6 ? R(sMY[-3 * KY]) : R(0.0), Y_p3 = W6 ? R(sMY[3 * KY]) : R(0.0);
                     const R qYn = vN * ip6<S>(vN, Y_m2, Y_m1, Y_00, Y_p1, Y_p2, Y_p3) + nYn;
                     const R qYs = vS * ip6<S>(vS, Y_m3, Y_m2, Y_m1, Y_00, Y_p1, Y_p2) + nYs;
-                    advch = -((qXe - qXw) * rcdx + (qYn - qYs) * R(rfdy));
+                    dX = qXe - qXw;
+                    dY = qYn - qYs;
                     return gd.bad() && vb;
                 };
                 if (fluxes(std::true_type{})) {
@@ -620,11 +635,11 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                 }
                 const R q_km = below(q_k, C_QV);
                 if (vb && j <= g.JEH) {
-                    const R advcv = -(q_k - q_km) * R(rcdz_L);
+                    const R adv = advection(q_k - q_km, R(rcdz_L), dX, rcdx, dY, R(rfdy));
                     const double pg = (dpn - dpc[1]) * rfdy;
                     const R cf = cor_v * (R(sMX[KY]) + R(sMX[0]) + R(sMX[KY - KX]) + R(sMX[-KX]));
                     const R div = !use_div ? R(0.0) : ddc * (ld(a.DDIV + c + sJ) - ld(a.DDIV + c)) * fdy;
-                    const double val = V0 + dt * (((((double)(advcv + advch)) - pg) + (double)cf) + (double)div + (double)tV);
+                    const double val = V0 + dt * (((((double)adv) - pg) + (double)cf) + (double)div + (double)tV);
                     fold_state<M>(a, ptr, N3, 3, a.MOMY_RK, a.MOMY0, c, val, V0, aV);
                 }
             }
