@@ -16,7 +16,11 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <type_traits>
+
 #include <cuda_runtime.h>
+
+#include "rn_div.cuh"
 
 namespace hevi {
 
@@ -144,8 +148,14 @@ __device__ __forceinline__ R koren_phi(R v1, R v2, R v3)
     const R eps = R(EPS);
     const R zerosw1 = eps - fsign(eps, fabs(v1 - v2) - eps);
     const R zerosw2 = eps - fsign(eps, fabs(v2 - v3) - eps);
-    const R r2 = R(2.0) * (v1 - v2 + zerosw1 * zerosw2) / (v2 - v3 + zerosw2);
-    return rmax(R(0.0), rmin(r2, rmin((R(1.0) + r2) / R(3.0), R(2.0))));
+    if constexpr (std::is_floating_point_v<R>) {
+        // (a zero r2 may have the other sign than with `/`; the value it limits is unchanged)
+        const R r2 = rn::quotient_mag(R(2.0) * (v1 - v2 + zerosw1 * zerosw2), v2 - v3 + zerosw2);
+        return rmax(R(0.0), rmin(r2, rmin(rn::third(R(1.0) + r2), R(2.0))));
+    } else {
+        const R r2 = R(2.0) * (v1 - v2 + zerosw1 * zerosw2) / (v2 - v3 + zerosw2);
+        return rmax(R(0.0), rmin(r2, rmin((R(1.0) + r2) / R(3.0), R(2.0))));
+    }
 }
 
 // ---- face interpolation of the flux schemes ----------------------------------
@@ -167,6 +177,17 @@ __device__ __forceinline__ R ip4(R vel, R vm1, R v0, R vp1, R vp2)
     } else if constexpr (S == CD2) {
         return R(0.5) * (vp1 + v0);
     } else {
+        if constexpr (std::is_floating_point_v<R>) {
+            // The side that the flow does not come from enters times zero: with finite
+            // values (and no difference of them out of range) only the upwind side is formed.
+            // A tracer step at 250x190x77 without FCT, bound by its 24 quotients a cell:
+            // 651 -> 518 us with half of them, and without the compiler's division.
+            if (fabs(vm1) + fabs(v0) + fabs(vp1) + fabs(vp2) < R(1e30)) {
+                const bool up = fsign(R(0.5), vel) > R(0.0);
+                const R b = up ? v0 : vp1, dn = up ? vp1 : v0, far = up ? vm1 : vp2;
+                return b + R(0.5) * koren_phi(dn, b, far) * (b - far);
+            }
+        }
         return (v0 + R(0.5) * koren_phi(vp1, v0, vm1) * (v0 - vm1)) * (R(0.5) + fsign(R(0.5), vel))
                + (vp1 + R(0.5) * koren_phi(v0, vp1, vp2) * (vp1 - vp2)) * (R(0.5) - fsign(R(0.5), vel));
     }
