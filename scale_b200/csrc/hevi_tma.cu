@@ -29,8 +29,8 @@
 // cannot move across: the quotients are straight-line code (rn_div.cuh), the RK
 // fold is a template parameter, and columns and levels beyond the domain run along
 // at clamped addresses and only their stores are masked. 512x512x128, CD4, FP64:
-// 5.85 -> 4.45 ms per stage (402 instead of 640 million warp instructions on a
-// quarter of it, and 54% instead of 33% of DRAM peak).
+// 5.70 -> 4.29 ms per launch, the mean of a step's four (on 256x256x128 402 instead of
+// 640 million warp instructions, and 54% instead of 33% of DRAM peak).
 //
 // Every value keeps the operation order of the fused kernel k_hevi_stage
 // (hevi_stage.cu) and of the reference, so the two forms give identical bits.
@@ -53,6 +53,14 @@ template <int S> __host__ __device__ constexpr int box_k() { return wide_scheme(
 template <int S> __host__ __device__ constexpr int box_w() { return TX + 2 * reach<S>(); }
 template <int S> __host__ __device__ constexpr int box_h() { return TY + 2 * reach<S>(); }
 template <int S> __host__ __device__ constexpr int plane() { return box_k<S>() * box_w<S>() * box_h<S>(); }
+// Split march: a CTA takes one chunk instead of the whole column. The lowest two lanes
+// of a chunk above the first are then levels of the chunk below, run along for the
+// z fluxes, Sr and St that the chunk's first level needs, so a chunk advances 30 levels.
+constexpr int NGHOST = 2;
+__host__ __device__ constexpr int chunks(int KMAX, bool split)
+{
+    return !split ? (KMAX + KC - 1) / KC : KMAX <= KC ? 1 : 1 + (KMAX - KC + KC - NGHOST - 1) / (KC - NGHOST);
+}
 constexpr int NF = 5;                         // staged fields
 enum StagedField : int { F_DN = 0, F_MZ = 1, F_MX = 2, F_MY = 3, F_RT = 4 };
 constexpr int NDP = 33;                       // levels of a chunk's level tables: L0-1 .. L0+31
@@ -165,7 +173,7 @@ __device__ __forceinline__ void rim_flux(const StageArgsT<R> &a, const StagePtrs
 template <int S, typename R, int M, int LD, int NM>
 __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
     k_hevi_explicit(const Grid gt, const StageArgsT<R> a, const BatchT<NM> B, const __grid_constant__ StagePtrs<R> ptr,
-                    const __grid_constant__ StateMaps maps)
+                    const bool split, const __grid_constant__ StateMaps maps)
 {
     constexpr int H = reach<S>(), BW = box_w<S>(), BK = box_k<S>(), PL = plane<S>();
     constexpr int KX = BK, KY = BW * BK; // shared-memory strides of one column step in i and in j
@@ -184,6 +192,11 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
     const Grid g = block_domain(gt, B, b);
     const int lane = threadIdx.x, w = threadIdx.y, tid = w * 32 + lane;
     const int tx = w % TX, ty = w / TX;
+    // the chunks of this CTA: all of the column's, or one of the split march's
+    const int KST = split ? KC - NGHOST : KC, ns = chunks(g.KMAX, split);
+    const int ch0 = split ? b % ns : 0, ch1 = split ? ch0 + 1 : ns;
+    if (split) b /= ns;
+    const int ghosts = ch0 > 0 ? NGHOST : 0; // lanes below the chunk's own levels
     int ti, tj;
     {
         // raster: consecutive CTAs walk down a.raster rows of tiles, then step in i
@@ -207,20 +220,19 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
     const R ddc = use_div ? R(a.divdmp_coef / dt) : R(0.0);
     const R h = R(0.5), qr = R(0.25), J33R = R(J33G);
     const unsigned FULL = 0xffffffffu;
-    const int NC = (g.KMAX + KC - 1) / KC;
 
     // the chunk's box: levels L0-4 .., columns i0-H .., rows j0-H .. of every staged field
     auto issue = [&](int ch) {
         if constexpr (LD == LD_TMA) {
             if (tid != 0) return;
-            // box origin (0-based): level L0-4 = 32*ch - 2 (even, so its byte offset is a
+            // box origin (0-based): level L0-4 = KST*ch - 2 (even, so its byte offset is a
             // multiple of 16), column i0-H, row j0-H
-            const int x = KC * ch + (KS - 1) - KLO, y = i0 - H - 1, z = j0 - H - 1;
+            const int x = KST * ch + (KS - 1) - KLO, y = i0 - H - 1, z = j0 - H - 1;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_expect_tx(bar, (unsigned)(NF * PL * sizeof(double)));
             for (int f = 0; f < NF; ++f) tma_load_3d(stg + f * PL, &maps.m[f], x, y, z, bar);
         } else {
-            const int l0 = KS + KC * ch - KLO; // the level of box element 0
+            const int l0 = KS + KST * ch - KLO; // the level of box element 0
             constexpr int TAIL = BK - 32;      // levels of a column beyond one per lane
             for (int q = w; q < BW * BW; q += NCOL) {
                 const int ii = i0 - H + q % BW, jj = j0 - H + q / BW;
@@ -243,7 +255,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    issue(0);
+    issue(ch0);
     __syncthreads();
 
     // this warp's column in the staged box, at the lane's level of the chunk
@@ -279,11 +291,11 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
     };
     enum { C_MZ, C_TZ, C_SR, C_ST, C_QW, C_QU, C_QV };
 
-    for (int ch = 0; ch < NC; ++ch) {
-        const int L0 = KS + KC * ch, L = L0 + lane;
+    for (int ch = ch0; ch < ch1; ++ch) {
+        const int L0 = KS + KST * ch, L = L0 + lane;
         const int lev = min(L, KE) - 1;  // lanes above KE run along on the last level
         const int c = col + lev, cs = cside + lev;
-        const bool vb = col_ok && L <= KE;
+        const bool vb = col_ok && L <= KE && lane >= ghosts;
 
         // ---- a. DPRES (:355) at the chunk's levels of this warp's column and of its side
         // column, the level tables (levels L0-1..L0+31, clamped to KE), RHOT -> POTT.
@@ -292,9 +304,9 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
         double rt_s = 0.0, dp0_s = 0.0, rr_s = 0.0;
         if (side) { rt_s = ld(a.RT2P + cs); dp0_s = ld(a.DPRES0 + cs); rr_s = ld(a.REF_rhot + cs); }
         if constexpr (LD == LD_TMA) {
-            if (!mbar_wait(bar, ch & 1)) { // bounded; the block leaves at the barrier below
+            if (!mbar_wait(bar, (ch - ch0) & 1)) { // bounded; the block leaves at the barrier below
                 s_ok = 0;
-                (void)mbar_wait(bar, ch & 1); // bounded: the copies still in flight
+                (void)mbar_wait(bar, (ch - ch0) & 1); // bounded: the copies still in flight
             }
         } else {
             copy_wait();
@@ -469,7 +481,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                 const R tW = lds(a.MOMZ_t + ck);
                 const R Sr_k = below(Sr, C_SR), St_k = below(St, C_ST);
                 const int k = L - 1;
-                const bool vc = col_ok && (!EDGE || (k >= KS && k <= KE - 1));
+                const bool vc = col_ok && lane >= ghosts && (!EDGE || (k >= KS && k <= KE - 1));
                 const double *cMZ = sMZ - 1, *cDN = sDN - 1, *cMX = sMX - 1, *cMY = sMY - 1; // level k
                 R q_k, dX = R(0.0), dY = R(0.0);
                 auto fluxes = [&](auto fast) {
@@ -657,7 +669,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
 #undef fdz_k
 #undef wd_k
         __syncthreads(); // every read of the staged box and of DPRES is done
-        if (ch + 1 < NC) issue(ch + 1);
+        if (ch + 1 < ch1) issue(ch + 1);
     }
 }
 
@@ -676,8 +688,9 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
 // The solve's serial chain and the update's 13 to 18 streams bound it in turn: of
 // about 115 thousand cycles of a CTA at 128 levels the solve took 57 and the update 45
 // (a level 400 cycles, most of it waiting for its operands' shared-memory reads).
-// 512x512x128, CD4, FP64: stage 6.35 -> 5.9 ms with the operands read ahead and the
-// combine's state sums formed from the stage buffers instead of accumulated.
+// 512x512x128, CD4, FP64: 2.00 -> 1.52 ms per launch, the mean of a step's four, with the
+// operands read ahead and the combine's state sums formed from the stage buffers
+// instead of accumulated.
 constexpr int CCOLS = 16;  // columns per CTA (consecutive in i)
 constexpr int CWARPS = 8;
 __host__ __device__ inline int col_pitch_c(int KA) { return KA | 1; }
@@ -899,6 +912,32 @@ __global__ void __launch_bounds__(32 * CWARPS, 4)
 // =============================================================================
 // host side
 // =============================================================================
+inline long long tiles(const Grid &m) { return (long long)((m.IMAX + TX - 1) / TX) * ((m.JMAX + TY - 1) / TY); }
+
+// Whether the explicit kernel splits the march: where that shortens the time of the
+// last CTA, counted in chunks, with 148 SMs of `per_sm` CTAs. A CTA that marches takes
+// its chunks one after another, so a domain of few tiles leaves most of the chip idle
+// (40x40x80: 100 CTAs of 3 chunks against 300 of one), and one of a few waves ends in a
+// nearly empty one; the split takes more chunks in deep columns, for the ghost levels.
+// Marching against split: 40x40x80, UD3 (3 chunk times against 2), 40 and 31 us per launch,
+// a short step 290 and 256 us; 253x187x57, UD3 (22 against 21), a step 2773 and 2700 us;
+// 512x512x128, CD4 (224 against 277), 25.9 and 26.8 ms; a stage at 200x136x64, UD5
+// (24 against 35), 360 and 476 us. FP64 only: the split moves levels between the code
+// with and without wall forms, whose FP32 sums the compiler may fuse differently.
+inline bool split_march(const Grid &g, const Members &mem, int per_sm)
+{
+    long long whole = 0, parts = 0, longest = 0;
+    for (int q = 0; q < (mem.n > 1 ? mem.n : 1); ++q) {
+        const Grid m = mem.n > 1 ? member_grid(g, mem.m[q]) : g;
+        whole += tiles(m) * chunks(m.KMAX, false);
+        parts += tiles(m) * chunks(m.KMAX, true);
+        longest = chunks(m.KMAX, false) > longest ? chunks(m.KMAX, false) : longest;
+    }
+    const long long slots = 148LL * per_sm;
+    const long long marched = (whole + longest * slots - 1) / (longest * slots) * longest;
+    return (parts + slots - 1) / slots < marched;
+}
+
 // the two kernels over the blocks of every member
 template <int S, int M, int LD, int NM, typename R>
 cudaError_t launch_pair(const Grid &g, const Members &mem, const StageArgsT<R> &a, const StageMaps<R> &h, cudaStream_t st)
@@ -923,8 +962,9 @@ cudaError_t launch_pair(const Grid &g, const Members &mem, const StageArgsT<R> &
     auto kx = k_hevi_explicit<S, R, M, LD, NM>;
     cudaError_t e = open_smem(kx, smem_bytes<S>());
     if (e != cudaSuccess) return e;
-    if (!ranges([](const Grid &m) { return ((m.IMAX + TX - 1) / TX) * ((m.JMAX + TY - 1) / TY); })) return cudaErrorInvalidValue;
-    kx<<<B.first[B.n], dim3(32, NCOL), smem_bytes<S>(), st>>>(g, a, B, h.ptr, h.maps);
+    const bool split = sizeof(R) == 8 && split_march(g, mem, wide_scheme(S) ? 1 : 2);
+    if (!ranges([&](const Grid &m) { return tiles(m) * (split ? chunks(m.KMAX, true) : 1); })) return cudaErrorInvalidValue;
+    kx<<<B.first[B.n], dim3(32, NCOL), smem_bytes<S>(), st>>>(g, a, B, h.ptr, split, h.maps);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     auto kc = k_hevi_column<R, M, NM>;
     // the attribute is set once per device, so it opens the largest size (KA = 260)
