@@ -30,6 +30,7 @@
 #include <cstdio>
 
 #include "hevi_kernels.cuh"
+#include "tma_util.cuh"
 #include "adjoint.cuh"
 
 namespace hevi {
@@ -720,7 +721,7 @@ __device__ void column_forward(IO &io, const Ctx &x, int i, int j)
 }
 
 template <int S, class IOT>
-__global__ void __launch_bounds__(128) k_column(const Ctx x)
+__global__ void __launch_bounds__(128) k_column(const __grid_constant__ Ctx x)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= x.g.IMAX * x.g.JMAX) return;
@@ -729,111 +730,186 @@ __global__ void __launch_bounds__(128) k_column(const Ctx x)
     column_forward<S>(io, x, i, j);
 }
 
-// adjoint of the column (values of PT, F1..F3 and C from the forward column);
-// adjoints are added with plain stores: this thread alone touches its column
+// The forward column and its adjoint take a warp per column: everything but the two
+// recurrences runs with its lanes along k (one thread per column read and wrote
+// columns KA doubles apart, 16384 threads on the whole chip at 128x128), the
+// recurrences in shared memory by lane 0. 128x128x64, CD4: the forward column
+// 214 -> 85 us, the adjoint one 688 -> 127 us; an adjoint step 9.67 -> 5.63 ms with the
+// reverse sweep's shorter recomputation (stage_fwd). Eight columns per CTA with their
+// recurrences on eight lanes of one warp measured the same.
+constexpr int CW = 4; // columns (warps) per CTA
+constexpr int FWD_ARRAYS = 5, ADJ_ARRAYS = 6;
+inline size_t column_smem(int KA, int arrays) { return (size_t)CW * arrays * KA * sizeof(double); }
+
+// hevi_solver :665-809, as column_forward in FP64
 template <int S>
-__global__ void __launch_bounds__(128) k_column_adj(const Ctx x)
+__global__ void __launch_bounds__(32 * CW) k_column_warp(const __grid_constant__ Ctx x)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= x.g.IMAX * x.g.JMAX) return;
+    extern __shared__ double sh[];
     const Grid &g = x.g;
-    const int i = g.IS + t % g.IMAX, j = g.JS + t / g.IMAX;
-    const int KS = g.KS, KE = g.KE;
+    const int t = blockIdx.x * CW + threadIdx.y, lane = threadIdx.x;
+    if (t >= g.IMAX * g.JMAX) return; // warp-uniform
+    const int i = g.IS + t % g.IMAX, j = g.JS + t / g.IMAX, KS = g.KS, KE = g.KE;
+    const size_t c1 = idx3(g, 1, i, j);
+    auto C_ = [&](int k) { return c1 + (size_t)(k - 1); };
+    double *P = sh + (size_t)threadIdx.y * FWD_ARRAYS * g.KA - 1; // 1-based level index
+    double *F1 = P + g.KA, *F2 = F1 + g.KA, *F3 = F2 + g.KA, *C = F3 + g.KA;
+    const double dt = x.dt, J33G = x.J33G, dt2 = dt * dt;
+    FwdIO io(x);
+    auto in = [&](int f, int k) { return x.val[f][C_(k)]; };
+    auto out = [&](int f, int k, double v) { x.val[f][C_(k)] = v; };
+    for (int k = KS + lane; k <= KE - 1; k += 32) {
+        P[k] = face_theta<S>(io, x, C_(k), k);
+        out(PTf, k, P[k]);
+    }
+    __syncwarp();
+    auto Acoef = [&](int k) { return dt2 * J33G * ld(g.RCDZ + k - 1) * in(RT2P, k) * J33G; };
+    for (int k = KS + lane; k <= KE - 1; k += 32) {
+        const double rfdz = ld(g.RFDZ + k - 1);
+        const double B = GRAV * dt2 * J33G / (ld(g.CDZ + k) + ld(g.CDZ + k - 1));
+        const double Ak = Acoef(k), Ak1 = Acoef(k + 1);
+        // right-hand side C(k) (:698-722)
+        const double pg = -(in(DPRES, k + 1) + in(RT2P, k + 1) * dt * in(ST, k + 1) - in(DPRES, k) - in(RT2P, k) * dt * in(ST, k))
+                              * rfdz * J33G
+                          - GRAV * (ld(g.F2H1 + k - 1) * (in(XD, k + 1) - in(REFDENS, k + 1) + in(SR, k + 1) * dt)
+                                    + ld(g.F2H2 + k - 1) * (in(XD, k) - in(REFDENS, k) + in(SR, k) * dt));
+        C[k] = in(XW, k) + dt * (pg + in(SW, k));
+        F2[k] = 1.0 + (P[k] * rfdz * (Ak1 + Ak));
+        F1[k] = k <= KE - 2 ? -(P[k + 1] * rfdz * Ak1 + B) : 0.0;
+        F3[k] = k > KS ? -(P[k - 1] * rfdz * Ak - B) : 0.0;
+        out(F1f, k, F1[k]);
+        out(F2f, k, F2[k]);
+        out(F3f, k, F3[k]);
+    }
+    __syncwarp();
+    if (lane == 0) { // e replaces F1, f replaces C
+        double r = 1.0 / F2[KS], e = -F1[KS] * r, f = C[KS] * r;
+        F1[KS] = e;
+        C[KS] = f;
+        for (int k = KS + 1; k <= KE - 2; ++k) {
+            r = 1.0 / (F2[k] + F3[k] * e);
+            e = -F1[k] * r;
+            f = (C[k] - F3[k] * f) * r;
+            F1[k] = e;
+            C[k] = f;
+        }
+        f = (C[KE - 1] - F3[KE - 1] * f) / (F2[KE - 1] + F3[KE - 1] * e);
+        C[KE - 1] = f;
+        for (int k = KE - 2; k >= KS; --k) {
+            f = F1[k] * f + C[k];
+            C[k] = f;
+        }
+    }
+    __syncwarp();
+    // back-update :728-790
+    for (int m = KS + lane; m <= KE; m += 32) {
+        const double rcdz = ld(g.RCDZ + m - 1);
+        const double Cm = m <= KE - 1 ? C[m] : 0.0, Cm1 = m >= KS + 1 ? C[m - 1] : 0.0;
+        double adr, adt;
+        if (m == KE) {
+            adr = Cm1 * J33G * rcdz;
+            adt = Cm1 * P[KE - 1] * J33G * rcdz;
+        } else if (m == KS) {
+            adr = -Cm * J33G * rcdz;
+            adt = -Cm * P[KS] * J33G * rcdz;
+        } else {
+            adr = -(Cm - Cm1) * J33G * rcdz;
+            adt = -(Cm * P[m] - Cm1 * P[m - 1]) * J33G * rcdz;
+        }
+        if (m <= KE - 1) out(Cf, m, Cm);
+        out(ODRK, m, in(X0D, m) + dt * (adr + in(SR, m)));
+        out(ORRK, m, in(X0R, m) + dt * (adt + in(ST, m)));
+        out(OWRK, m, m <= KE - 1 ? in(X0W, m) + (Cm - in(XW, m)) : 0.0);
+        if (m == KS) out(OWRK, KS - 1, 0.0);
+    }
+}
+
+// adjoint of the column (values of PT, F1..F3 and C from the forward column).
+// Every level gathers what the rows k-1, k and k+1 give it; adjoints are added with
+// plain stores (this warp alone touches its column) but for the face theta's, whose
+// levels overlap
+template <int S>
+__global__ void __launch_bounds__(32 * CW) k_column_adj(const __grid_constant__ Ctx x)
+{
+    extern __shared__ double sh[];
+    const Grid &g = x.g;
+    const int t = blockIdx.x * CW + threadIdx.y, lane = threadIdx.x;
+    if (t >= g.IMAX * g.JMAX) return; // warp-uniform
+    const int i = g.IS + t % g.IMAX, j = g.JS + t / g.IMAX, KS = g.KS, KE = g.KE;
     const size_t c1 = idx3(g, 1, i, j);
     auto C_ = [&](int k) { return c1 + (size_t)(k - 1); };
     const double dt = x.dt, J33G = x.J33G, dt2 = dt * dt;
-    double *const *V = x.val;
-    double *const *L = x.aux;
-    auto val = [&](int f, int k) { return V[f][C_(k)]; };
-    auto lam = [&](int f, int k) -> double & { return L[f][C_(k)]; };
-    // adjoint of the solution C and of PT, gathered in the column work arrays
-    // (aux of Cf and PTf), then the transposed solve in Ef/Ff (values)
-    for (int k = KS - 1; k <= KE; ++k) {
-        lam(Cf, k) = 0.0;
-        lam(PTf, k) = 0.0;
+    auto val = [&](int f, int k) { return x.val[f][C_(k)]; };
+    auto lam = [&](int f, int k) -> double & { return x.aux[f][C_(k)]; };
+    double *F1 = sh + (size_t)threadIdx.y * ADJ_ARRAYS * g.KA - 1; // 1-based level index
+    double *F2 = F1 + g.KA, *F3 = F2 + g.KA, *C = F3 + g.KA, *P = C + g.KA, *Y = P + g.KA;
+    for (int k = KS + lane; k <= KE - 1; k += 32) {
+        F1[k] = val(F1f, k);
+        F2[k] = val(F2f, k);
+        F3[k] = val(F3f, k);
+        C[k] = val(Cf, k);
+        P[k] = val(PTf, k);
     }
-    for (int m = KS; m <= KE; ++m) {
-        const double rcdz = ld(g.RCDZ + m - 1);
-        const double lD = lam(ODRK, m), lR = lam(ORRK, m);
-        lam(X0D, m) += lD;
-        lam(X0R, m) += lR;
-        lam(SR, m) += dt * lD;
-        lam(ST, m) += dt * lR;
-        const double gD = dt * lD * J33G * rcdz, gR = dt * lR * J33G * rcdz;
-        if (m == KE) {
-            lam(Cf, KE - 1) += gD + gR * val(PTf, KE - 1);
-            lam(PTf, KE - 1) += gR * val(Cf, KE - 1);
-        } else if (m == KS) {
-            lam(Cf, KS) -= gD + gR * val(PTf, KS);
-            lam(PTf, KS) -= gR * val(Cf, KS);
-        } else {
-            lam(Cf, m) -= gD + gR * val(PTf, m);
-            lam(PTf, m) -= gR * val(Cf, m);
-            lam(Cf, m - 1) += gD + gR * val(PTf, m - 1);
-            lam(PTf, m - 1) += gR * val(Cf, m - 1);
-        }
-        if (m <= KE - 1) {
-            const double lW = lam(OWRK, m);
-            lam(X0W, m) += lW;
-            lam(Cf, m) += lW;
-            lam(XW, m) -= lW;
-        }
-    }
+    __syncwarp();
+    // adjoints of the density and theta updates at level m
+    auto gD = [&](int m) { return dt * lam(ODRK, m) * J33G * ld(g.RCDZ + m - 1); };
+    auto gR = [&](int m) { return dt * lam(ORRK, m) * J33G * ld(g.RCDZ + m - 1); };
+    // the adjoint of the solution C
+    for (int k = KS + lane; k <= KE - 1; k += 32)
+        Y[k] = (gD(k + 1) + gR(k + 1) * P[k]) - (gD(k) + gR(k) * P[k]) + lam(OWRK, k);
+    __syncwarp();
     // transposed tridiagonal solve: M^T y = lam(C). Row r of M (level k) holds
     // F3(k) C(k-1) + F2(k) C(k) + F1(k) C(k+1); M^T has F1(k-1) below the
-    // diagonal and F3(k+1) above it. Elimination factors in val(Ef), val(Ff).
-    {
+    // diagonal and F3(k+1) above it. The elimination factors replace F2 and Y.
+    if (lane == 0) {
         double cp = 0.0, bp = 0.0;
         for (int k = KS; k <= KE - 1; ++k) {
-            const double sub = k > KS ? val(F1f, k - 1) : 0.0;
-            const double sup = k < KE - 1 ? val(F3f, k + 1) : 0.0;
-            const double m = val(F2f, k) - sub * cp;
+            const double sub = k > KS ? F1[k - 1] : 0.0, sup = k < KE - 1 ? F3[k + 1] : 0.0;
+            const double m = F2[k] - sub * cp;
             cp = sup / m;
-            bp = (lam(Cf, k) - sub * bp) / m;
-            V[Ef][C_(k)] = cp;
-            V[Ff][C_(k)] = bp;
+            bp = (Y[k] - sub * bp) / m;
+            F2[k] = cp;
+            Y[k] = bp;
         }
         double y = bp;
-        lam(Ff, KE - 1) = y;
         for (int k = KE - 2; k >= KS; --k) {
-            y = V[Ff][C_(k)] - V[Ef][C_(k)] * y;
-            lam(Ff, k) = y; // lam(Ff) now holds y = the adjoint of the right-hand side
+            y = Y[k] - F2[k] * y;
+            Y[k] = y; // the adjoint of the right-hand side
         }
     }
-    auto Acoef = [&](int k) { return dt2 * J33G * ld(g.RCDZ + k - 1) * V[RT2P][C_(k)] * J33G; };
-    for (int k = KS; k <= KE - 1; ++k) {
-        const double y = lam(Ff, k);
-        const double rfdz = ld(g.RFDZ + k - 1);
-        const double Ak = Acoef(k), Ak1 = Acoef(k + 1);
-        // matrix entries: lam(M_rc) = -y_r C_c
-        const double lF2 = -y * val(Cf, k);
-        lam(PTf, k) += lF2 * rfdz * (Ak1 + Ak);
-        if (k <= KE - 2) lam(PTf, k + 1) -= (-y * val(Cf, k + 1)) * rfdz * Ak1;
-        if (k > KS) lam(PTf, k - 1) -= (-y * val(Cf, k - 1)) * rfdz * Ak;
+    __syncwarp();
+    auto Acoef = [&](int k) { return dt2 * J33G * ld(g.RCDZ + k - 1) * val(RT2P, k) * J33G; };
+    for (int k = KS + lane; k <= KE; k += 32) {
+        const double lD = lam(ODRK, k), lR = lam(ORRK, k);
+        const double y = k <= KE - 1 ? Y[k] : 0.0, ym = k > KS ? Y[k - 1] : 0.0;
+        const double rf = k <= KE - 1 ? ld(g.RFDZ + k - 1) : 0.0, rfm = k > KS ? ld(g.RFDZ + k - 2) : 0.0;
         // right-hand side C(k) = MOMZ(k) + dt (pg + Sw(k))
-        lam(XW, k) += y;
-        const double gy = dt * y;
-        lam(SW, k) += gy;
-        const double a = -gy * rfdz * J33G;
-        lam(DPRES, k + 1) += a;
-        lam(DPRES, k) -= a;
-        lam(ST, k + 1) += a * V[RT2P][C_(k + 1)] * dt;
-        lam(ST, k) -= a * V[RT2P][C_(k)] * dt;
-        const double b = -gy * GRAV;
-        const double f1 = ld(g.F2H1 + k - 1), f2 = ld(g.F2H2 + k - 1);
-        lam(XD, k + 1) += b * f1;
-        lam(SR, k + 1) += b * f1 * dt;
-        lam(XD, k) += b * f2;
-        lam(SR, k) += b * f2 * dt;
-    }
-    // face theta: PT(k) from POTT (the UD3 switch on MOMZ has no derivative)
-    for (int k = KS; k <= KE - 1; ++k) {
-        const double lpt = lam(PTf, k);
+        const double a0 = -(dt * y) * rf * J33G, am = -(dt * ym) * rfm * J33G, rt = val(RT2P, k);
+        const double b = -(dt * y) * GRAV * (k <= KE - 1 ? ld(g.F2H2 + k - 1) : 0.0)
+                         - (dt * ym) * GRAV * (k > KS ? ld(g.F2H1 + k - 2) : 0.0);
+        lam(X0D, k) += lD;
+        lam(X0R, k) += lR;
+        lam(DPRES, k) += am - a0;
+        lam(ST, k) += dt * lR + (am - a0) * rt * dt;
+        lam(XD, k) += b;
+        lam(SR, k) += dt * lD + b * dt;
+        if (k > KE - 1) continue;
+        const double lW = lam(OWRK, k);
+        lam(X0W, k) += lW;
+        lam(XW, k) += y - lW;
+        lam(SW, k) += dt * y;
+        // matrix entries: lam(M_rc) = -y_r C_c, at PT(k) from the rows k, k-1 (F1) and k+1 (F3)
+        const double Ak = Acoef(k), Ak1 = Acoef(k + 1), Ck = C[k];
+        double lpt = (gR(k + 1) - gR(k)) * Ck - y * Ck * rf * (Ak1 + Ak);
+        if (k > KS) lpt += ym * Ck * rfm * Ak;
+        if (k < KE - 1) lpt += Y[k + 1] * Ck * ld(g.RFDZ + k) * Ak1;
+        // face theta: PT(k) from POTT (the UD3 switch on MOMZ has no derivative)
         if (lpt == 0.0) continue;
         AdjIO<5> io(x);
         const Jet<5> pt = face_theta<S>(io, x, C_(k), k);
-        for (int q = 0; q < io.n; ++q)
-            if (pt.d[q] != 0.0) L[io.fid[q]][io.off[q]] += lpt * pt.d[q];
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+            if (q < io.n && pt.d[q] != 0.0) atomicAdd(x.aux[io.fid[q]] + io.off[q], lpt * pt.d[q]);
     }
 }
 
@@ -1113,8 +1189,12 @@ cudaError_t numfilter(Mode m, const Ctx &x, cudaStream_t st)
     return cudaSuccess;
 }
 
+// momenta: with the updates of rho*u and rho*v and their fluxes. The adjoint of a
+// stage needs none of these values (its passes are linear in the fluxes), so the
+// reverse sweep recomputes a stage without them: eight launches, 103 us of
+// 306, at 128x128x64, CD4.
 template <int S>
-cudaError_t stage_fwd(Mode m, const Ctx &x, cudaStream_t st)
+cudaError_t stage_fwd(Mode m, const Ctx &x, cudaStream_t st, bool momenta = true)
 {
     const Grid &g = x.g;
     const int KS = g.KS, KE = g.KE, IS = g.IS, IE = g.IE, JS = g.JS, JE = g.JE;
@@ -1132,11 +1212,17 @@ cudaError_t stage_fwd(Mode m, const Ctx &x, cudaStream_t st)
     RUN(run<PassST, 7>(m, x, Box{KS, KE, IS, IE, JS, JE}, st));
     {
         const int n = g.IMAX * g.JMAX;
-        if (m == M_TLM) k_column<S, TlmIO><<<(n + 127) / 128, 128, 0, st>>>(x);
-        else if (m == M_DD) k_column<S, DdIO><<<(n + 127) / 128, 128, 0, st>>>(x);
-        else k_column<S, FwdIO><<<(n + 127) / 128, 128, 0, st>>>(x);
+        if (m == M_TLM) {
+            k_column<S, TlmIO><<<(n + 127) / 128, 128, 0, st>>>(x);
+        } else if (m == M_DD) {
+            k_column<S, DdIO><<<(n + 127) / 128, 128, 0, st>>>(x);
+        } else {
+            RUN(tma::open_smem(k_column_warp<S>, column_smem(260, FWD_ARRAYS)));
+            k_column_warp<S><<<(n + CW - 1) / CW, dim3(32, CW), column_smem(g.KA, FWD_ARRAYS), st>>>(x);
+        }
         RUN(cudaGetLastError());
     }
+    if (!momenta) return cudaSuccess;
     RUN(run<PassQHZ<S, 0>, 12>(m, x, Box{KS - 1, KE, IS, IE, JS, JE}, st));
     RUN(run<PassQHA<S, 0>, 10>(m, x, Box{KS, KE, IS - 1, IE, JS, JE}, st));
     RUN(run<PassQHC<S, 0>, 12>(m, x, Box{KS, KE, IS, IE, JS - 1, JE}, st));
@@ -1165,7 +1251,8 @@ cudaError_t stage_adj(const Ctx &x, cudaStream_t st)
     RUN(run<PassQHZ<S, 0>, 12>(m, x, Box{KS - 1, KE, IS, IE, JS, JE}, st));
     {
         const int n = g.IMAX * g.JMAX;
-        k_column_adj<S><<<(n + 127) / 128, 128, 0, st>>>(x);
+        RUN(tma::open_smem(k_column_adj<S>, column_smem(260, ADJ_ARRAYS)));
+        k_column_adj<S><<<(n + CW - 1) / CW, dim3(32, CW), column_smem(g.KA, ADJ_ARRAYS), st>>>(x);
         RUN(cudaGetLastError());
     }
     RUN(run<PassST, 7>(m, x, Box{KS, KE, IS, IE, JS, JE}, st));
@@ -1368,14 +1455,12 @@ static cudaError_t step_adj_impl(const Model &M, const double *X_in, double *lam
         bind_state(x, ODRK, b.xs_v + (size_t)s * 5 * N3, with_adj ? b.xs_a + (size_t)s * 5 * N3 : nullptr, N3);
         x.dt = dts[s];
     };
-    for (int s = 0; s < 4; ++s) {
+    for (int s = 0; s < 3; ++s) { // the inputs of the stages
         bind_stage(s, false);
         RUN(stage_fwd<S>(M_FWD, x, st));
-        if (s < 3) {
-            double *f[5];
-            for (int q = 0; q < 5; ++q) f[q] = b.xs_v + ((size_t)s * 5 + q) * N3;
-            periodic_halo(M.g, one, f, 5, st);
-        }
+        double *f[5];
+        for (int q = 0; q < 5; ++q) f[q] = b.xs_v + ((size_t)s * 5 + q) * N3;
+        periodic_halo(M.g, one, f, 5, st);
     }
     // ---- reverse sweep ----
     // lam holds the adjoint of the state after the step: move it to the
@@ -1404,7 +1489,7 @@ static cudaError_t step_adj_impl(const Model &M, const double *X_in, double *lam
     for (int s = 3; s >= 0; --s) {
         // forward values of this stage's intermediates, then its adjoint
         bind_stage(s, false);
-        RUN(stage_fwd<S>(M_FWD, x, st));
+        RUN(stage_fwd<S>(M_FWD, x, st, false));
         bind_stage(s, true);
         RUN(cudaMemsetAsync(b.inter_a, 0, (size_t)(N_INTER + 7) * N3 * sizeof(double), st));
         RUN(stage_adj<S>(x, st));
