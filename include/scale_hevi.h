@@ -487,9 +487,10 @@ int scale_hevi_ensemble_layout(long long *cell0, long long *col0, long long *z0,
     const double *ND_COEF, const double *ND_SFC_FACT, const double *dt
 
 /* The numerical filter's form for one domain (no counterpart in the
- * reference): 1, the default after setup, forms num_diff from tiles of the
- * filtered quantities staged in shared memory by bulk tensor copies wherever
- * the arrays admit tensor maps (16-byte aligned bases and strides); 0 keeps the
+ * reference), and of an ensemble's: 1, the default after setup, forms num_diff
+ * from tiles of the filtered quantities staged in shared memory, by bulk tensor
+ * copies where one domain's arrays admit tensor maps (16-byte aligned bases and
+ * strides) and by asynchronous copies elsewhere (ND_ORDER 1); 0 keeps the
  * column kernel. The results are identical. */
 int scale_hevi_numfilter_form(int tiled);
 

@@ -29,8 +29,8 @@
 // cannot move across: the quotients are straight-line code (rn_div.cuh), the RK
 // fold is a template parameter, and columns and levels beyond the domain run along
 // at clamped addresses and only their stores are masked. 512x512x128, CD4, FP64:
-// 5.70 -> 4.29 ms per launch, the mean of a step's four (on 256x256x128 402 instead of
-// 640 million warp instructions, and 54% instead of 33% of DRAM peak).
+// 5.70 -> 4.29 ms per launch, the mean of a step's four (on 256x256x128 405 instead of
+// 640 million warp instructions, and 44% instead of 33% of DRAM peak).
 //
 // Every value keeps the operation order of the fused kernel k_hevi_stage
 // (hevi_stage.cu) and of the reference, so the two forms give identical bits.
