@@ -90,8 +90,9 @@ __device__ __forceinline__ R zface_in(R vel, int m, const V &v)
 }
 
 // -(dq r) - (A a + B b), a momentum's vertical and horizontal flux divergence. FP64
-// code never fuses; FP32 code fuses A a into the horizontal sum and nothing else, whatever
-// else the compiler sees around it (the fused stage kernel's rounding)
+// code never fuses. FP32 code fuses A a into the horizontal sum and nothing else; left to
+// the compiler, what fuses depends on the code around it, and a mixed step's momenta
+// move by 1e-8 with it.
 __device__ __forceinline__ double advection(double dq, double r, double A, double a, double B, double b)
 {
     return -dq * r + -(A * a + B * b);
