@@ -296,7 +296,8 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
         const int L0 = KS + KST * ch, L = L0 + lane;
         const int lev = min(L, KE) - 1;  // lanes above KE run along on the last level
         const int c = col + lev, cs = cside + lev;
-        const bool vb = col_ok && L <= KE && lane >= ghosts;
+        const bool vl = col_ok && L <= KE; // a level of the domain, ghosts included
+        const bool vb = vl && lane >= ghosts;
 
         // ---- a. DPRES (:355) at the chunk's levels of this warp's column and of its side
         // column, the level tables (levels L0-1..L0+31, clamped to KE), RHOT -> POTT.
@@ -582,7 +583,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                                               R(sMX[KY]), W6 ? R(sMX[2 * KY]) : R(0.0)) + nYs;
                     dX = qXe - qXw;
                     dY = qYn - qYs;
-                    return gd.bad() && vb;
+                    return gd.bad() && vl; // a ghost lane hands its q_k on
                 };
                 if (fluxes(std::true_type{})) {
                     cold();
@@ -640,7 +641,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
                     const R qYs = vS * ip6<S>(vS, Y_m3, Y_m2, Y_m1, Y_00, Y_p1, Y_p2) + nYs;
                     dX = qXe - qXw;
                     dY = qYn - qYs;
-                    return gd.bad() && vb;
+                    return gd.bad() && vl; // a ghost lane hands its q_k on
                 };
                 if (fluxes(std::true_type{})) {
                     cold();
