@@ -510,19 +510,24 @@ int scale_hevi_persistent_wait(const double *seconds, const int *extra_arrivals)
 int scale_hevi_persistent_grid(int *ctas);
 
 /* ---------------------------------------------------------------------------
- * Launch shape of the stage kernel; no counterpart in the reference. A CTA
- * owns 16 columns as a tile of tile_x x (16/tile_x) columns (tile_x one of
- * 16, 8, 4) and CTAs are issued in raster groups of `raster` tile rows.
- * 0 selects the default (16, 16). The shape changes the speed only: results
- * are identical for every shape.
+ * Form and launch shape of the stage; no counterpart in the reference.
+ * tile_x = 0, the default, takes the tiled form (two kernels on 4 x 4 column
+ * tiles) wherever it applies: every domain and every FP64 ensemble. tile_x
+ * 16, 8 or 4 takes the fused kernel, whose CTA owns 16 columns as a tile of
+ * tile_x x (16/tile_x); a mixed-precision ensemble has it alone (width 16 for
+ * tile_x = 0). CTAs are issued in raster groups of `raster` tile rows (0: 16).
+ * The shape changes the speed only: FP64 results are identical for every
+ * shape; FP32 arithmetic may round differently in the two forms.
  * ------------------------------------------------------------------------- */
 int scale_hevi_stage_shape(int tile_x, int raster);
 /* Autotuner of that shape. With enable != 0, the next short-step call of each
- * path (FP64, mixed precision) outside a graph capture first times every
- * compiled tile width at raster heights 4, 16 and 64 on its own inputs (a
- * plain stage per candidate, outputs to library scratch; the caller's arrays
- * are not written) and keeps the fastest. scale_hevi_stage_shape() replaces
- * the choice and turns the tuner off. */
+ * path (FP64, mixed precision) outside a graph capture first times the tiled
+ * form, where it applies, and every width of the fused kernel at raster
+ * heights 4, 16 and 64 (the fused widths at 4 and 16 for an ensemble that has
+ * the tiled form) on its own inputs (a plain stage per candidate, outputs to
+ * library scratch; the caller's arrays are not written) and keeps the
+ * fastest. scale_hevi_stage_shape() replaces the choice and turns the tuner
+ * off. */
 int scale_hevi_stage_autotune(int enable);
 /* The shape in use on the FP64 (mixed = 0) or mixed-precision path. */
 int scale_hevi_stage_shape_get(int *tile_x, int *raster, int mixed);

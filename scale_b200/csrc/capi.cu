@@ -525,7 +525,10 @@ StageArgsT<F> stage_args(const StageInT<F> &in, double *const out[5], F *mflx, F
 // compiled tile width of the fused kernel, each at three raster heights, on
 // the caller's own inputs (one plain stage whose outputs go to the library's
 // scratch: the RK buffer, the flux RK sums, the column scratch; nothing the
-// caller holds is written) and keeps the fastest for this path.
+// caller holds is written) and keeps the fastest for this path. An ensemble that
+// has the tiled form times the fused widths at two of the heights: 64 was the slowest
+// or next to it for every width on the 48-member one (37.9, 37.6, 37.1 ms a stage for
+// 16, 8 and 4 wide, the best of 4 and 16 36.9, 36.7, 36.5).
 template <typename F>
 int autotune_stage(const StageInT<F> &in, double dtrk)
 {
@@ -542,15 +545,17 @@ int autotune_stage(const StageInT<F> &in, double dtrk)
     float best_ms = 1e30f;
     std::string rows;
     int rc = SCALE_HEVI_OK;
+    bool tiled_form = false;
     constexpr int FORMS[4] = {0, STAGE_TILE_XS[0], STAGE_TILE_XS[1], STAGE_TILE_XS[2]};
     for (int tx : FORMS) {
-        if (tx == 0 && C.members.size() > 1) continue; // an ensemble's shapes are those of the fused kernel
         for (int r : RASTERS) {
+            if (tx != 0 && r == RASTERS[2] && tiled_form && C.members.size() > 1) continue;
             const StageShape sh{tx, r};
             int nl = 1;
             bool tiled = false;
             cudaError_t e = launch_hevi_stage(C.g, mem(), a, C.scheme, sh, C.stream, &nl, &tiled); // warm-up
             if (e == cudaSuccess && tx == 0 && !tiled) break; // the tiled stage does not apply here
+            tiled_form |= tiled;
             cudaEventRecord(e0, C.stream);
             for (int q = 0; q < REPS && e == cudaSuccess; ++q) e = launch_hevi_stage(C.g, mem(), a, C.scheme, sh, C.stream);
             cudaEventRecord(e1, C.stream);

@@ -130,6 +130,27 @@ def test_autotuned_shape_gives_identical_results(cases, alone):
     assert min(c[2] for c in rep["candidates"]) == rep["chosen"][2]
 
 
+def test_autotuner_times_the_tiled_form_of_an_ensemble(cases, alone):
+    """The form an FP64 ensemble runs without tuning is among the tuner's candidates,
+    beside every tile width of the fused kernel; a mixed-precision ensemble has the
+    fused kernel only."""
+    for mixed in (False, True):
+        e = Ensemble(cases, mixed=mixed)
+        try:
+            hevi.stage_autotune(True)
+            e.run(NSTEPS)
+            got = e.members()
+            rep = hevi.autotune_report()
+            shape = hevi.stage_shape_get(mixed)
+        finally:
+            e.close()
+        assert {c[0] for c in rep["candidates"]} == ({16, 8, 4} if mixed else {0, 16, 8, 4})
+        assert rep["chosen"] == min(rep["candidates"], key=lambda c: c[2])
+        assert list(shape) == rep["chosen"][:2]
+        if not mixed:
+            _same(got, alone)
+
+
 @pytest.mark.parametrize("scheme", ["UD5", "CD6"])
 def test_six_point_ensemble_matches_members_alone(scheme):
     # members on a lateral halo of 3, advanced together and alone
