@@ -145,7 +145,9 @@ def test_autotuner_times_the_tiled_form_of_an_ensemble(cases, alone):
         finally:
             e.close()
         assert {c[0] for c in rep["candidates"]} == ({16, 8, 4} if mixed else {0, 16, 8, 4})
-        assert rep["chosen"] == min(rep["candidates"], key=lambda c: c[2])
+        # (the report rounds the times, so two candidates may show the same)
+        assert rep["chosen"] in rep["candidates"]
+        assert rep["chosen"][2] == min(c[2] for c in rep["candidates"])
         assert list(shape) == rep["chosen"][:2]
         if not mixed:
             _same(got, alone)
