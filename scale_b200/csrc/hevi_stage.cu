@@ -251,6 +251,7 @@ cudaError_t launch_hevi_stage(const Grid &g, const Members &mem, const StageArgs
         const cudaError_t e = launch_hevi_stage_tiled(g, mem, a, scheme, shape.raster, st);
         if (e != cudaErrorNotSupported) {
             if (tiled) *tiled = true;
+            if (launches) *launches = 2; // the explicit and the column kernel
             return e;
         }
     }

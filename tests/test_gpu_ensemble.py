@@ -89,6 +89,14 @@ def test_ensemble_one_launch_per_kernel(cases):
     assert l4 == l1
 
 
+@pytest.mark.parametrize("members", [1, 4])
+def test_tiled_stage_counts_both_of_its_kernels(cases, members):
+    # four stages a step; the fused form is one kernel per stage, the tiled form two
+    _, tiled = _together(cases[:members], 2)
+    _, fused = _together(cases[:members], 2, tile_x=16)
+    assert tiled - fused == 2 * 4
+
+
 def test_ensemble_mixed_precision_matches_members_alone(cases):
     # the FP32 arithmetic compiles with FMA contraction, which each kernel form
     # applies to its own code; the members alone take the fused form, as the
