@@ -60,7 +60,7 @@ struct Ctx {
     double *rk[3] = {nullptr, nullptr, nullptr}; // stage buffers, 5*N3 each
     double *facc = nullptr;         // 6*N3
     double *colscr = nullptr;       // 4*N3: Sr, St, tZ (fused and tiled stage), PT (tiled stage)
-    double *colC = nullptr;         // 2*N3: the column problem's right-hand side, then f, and e (tiled stage)
+    double *colC = nullptr;         // N3: the column problem's right-hand side (tiled stage)
     double *phi = nullptr;          // numerical filter: 5*N3 (allocated on first use)
     double *ndw = nullptr;          // numerical filter at ND_ORDER > 1: 2 x 15*N3 work (on first use)
     // mixed-precision path (allocated on first use): flux RK sums, column-solve
@@ -343,12 +343,7 @@ int use_metrics(const double *GSQRT, const double *J13G, const double *J23G, con
     }
     if (!C.tw_buf) {
         CK(dalloc(&C.tw_buf, (size_t)TERRAIN_WORK_FIELDS * C.N3));
-        double *q = C.tw_buf;
-        double **f[TERRAIN_WORK_FIELDS] = {&C.tw.POTT, &C.tw.DPRES, &C.tw.qZ, &C.tw.qX, &C.tw.qY, &C.tw.qJ13, &C.tw.qJ23,
-                                           &C.tw.Sr, &C.tw.Sw, &C.tw.St, &C.tw.mZ, &C.tw.mX, &C.tw.mY, &C.tw.tZ,
-                                           &C.tw.tX, &C.tw.tY, &C.tw.A, &C.tw.PT, &C.tw.F1, &C.tw.F2, &C.tw.F3,
-                                           &C.tw.C, &C.tw.e, &C.tw.f};
-        for (int q2 = 0; q2 < TERRAIN_WORK_FIELDS; ++q2) *f[q2] = q + (size_t)q2 * C.N3;
+        C.tw.bind(C.tw_buf, C.N3);
     }
     C.terrain = true;
     return SCALE_HEVI_OK;
@@ -910,7 +905,7 @@ int scale_hevi_ensemble_setup(int n, const scale_hevi_index *idx, const char *fl
         (rc = dalloc(&C.d_nd, 18 * (size_t)ZT + 18 * (size_t)XT + 18 * (size_t)YT)) ||
         (rc = dalloc(&C.rk[0], 5 * N3)) || (rc = dalloc(&C.rk[1], 5 * N3)) ||
         (rc = dalloc(&C.rk[2], 5 * N3)) || (rc = dalloc(&C.facc, 6 * N3)) ||
-        (rc = dalloc(&C.colscr, 4 * N3)) || (rc = dalloc(&C.colC, 2 * N3)) ||
+        (rc = dalloc(&C.colscr, 4 * N3)) || (rc = dalloc(&C.colC, N3)) ||
         (rc = dalloc(&C.sum_part, (size_t)x.IMAX * x.JMAX)) || (rc = dalloc(&C.sum_out, 1))) {
         free_all();
         return rc;

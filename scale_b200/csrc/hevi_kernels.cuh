@@ -62,13 +62,24 @@ __device__ __forceinline__ Block2 split_block(int b, int gx) { return {b % gx, b
 struct Metrics {
     const double *GSQRT, *J13G, *J23G, *MAPF, *PHI;
 };
-// work arrays of one field each (KA,IA,JA), device memory
+// Work arrays of one field each (KA,IA,JA), device memory. Nothing in them outlives a
+// stage, so those that only the HEVI stage uses share their memory with those that only
+// the HEVE stage uses.
+constexpr int TERRAIN_WORK_FIELDS = 13;
 struct TerrainWork {
-    double *POTT, *DPRES, *qZ, *qX, *qY, *qJ13, *qJ23, *Sr, *Sw, *St;
-    double *mZ, *mX, *mY, *tZ, *tX, *tY;
-    double *A, *PT, *F1, *F2, *F3, *C, *e, *f;
+    double *POTT, *DPRES, *mZ, *tZ;                          // both
+    double *Sr, *St, *PT, *F1, *F2, *F3, *C;                 // HEVI
+    double *qZ, *qX, *qY, *qJ13, *qJ23, *mX, *mY, *tX, *tY;  // HEVE
+    void bind(double *buf, size_t N3)
+    {
+        double **both[4] = {&POTT, &DPRES, &mZ, &tZ}, **hevi[7] = {&Sr, &St, &PT, &F1, &F2, &F3, &C};
+        double **heve[9] = {&qZ, &qX, &qY, &qJ13, &qJ23, &mX, &mY, &tX, &tY};
+        static_assert(TERRAIN_WORK_FIELDS == 4 + 9, "as many fields as the larger stage uses");
+        for (size_t q = 0; q < 4; ++q) *both[q] = buf + q * N3;
+        for (size_t q = 0; q < 7; ++q) *hevi[q] = buf + (4 + q) * N3;
+        for (size_t q = 0; q < 9; ++q) *heve[q] = buf + (4 + q) * N3;
+    }
 };
-constexpr int TERRAIN_WORK_FIELDS = 24;
 constexpr int TERRAIN_STAGE_LAUNCHES = 6; // kernels of one general-metric stage
 constexpr int TERRAIN_HEVE_LAUNCHES = 23;  // kernels of one general-metric HEVE stage
 cudaError_t launch_terrain_heve_stage(const Grid &g, const StageArgsT<double> &a, const Metrics &M,
