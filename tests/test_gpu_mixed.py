@@ -189,3 +189,59 @@ def test_mixed_numfilter_tiled_form_matches_column_form():
     for q in range(15):
         scale = np.max(np.abs(out[1][..., q]))
         assert np.max(np.abs(out[0][..., q] - out[1][..., q])) <= 1e-6 * max(scale, 1e-30), q
+
+
+# odd KMAX: no tensor maps, the stage and the filter stage their boxes with cp.async
+@pytest.mark.parametrize("scheme,kmax", [("UD3KOREN1993", 32), ("UD3KOREN1993", 33), ("UD3", 33), ("CD4", 33)],
+                         ids=lambda v: str(v))
+def test_mixed_precision_koren_and_odd_levels(scheme, kmax):
+    """100 short steps of a warm bubble, FP32 fluxes against FP64, to the bound of the
+    mixed path."""
+    g = mkinit.uniform_grid(32, 32, kmax, 200.0, 200.0, 200.0)
+    c = mkinit.make_case("mixed", g, scheme, scheme, dt=0.4, dtl=2.0,
+                         bubbles=[(3200.0, 3200.0, 2000.0, 1500.0, 1500.0, 1000.0, 2.0)], theta_noise=0.01, seed=7)
+    st64 = run_short_steps(c, 100, mixed=False)
+    st32 = run_short_steps(c, 100, mixed=True)
+    for n in STATE:
+        emax, erms = field_errors(st32[n], st64[n], c.g)
+        assert emax <= 1e-5, f"{n}: max {emax:.3e} rms {erms:.3e}"
+
+
+@pytest.mark.parametrize("fct,value", [(False, None), (False, 1e-20), (False, 1e29), (False, 1e31), (True, None),
+                                       (True, 1e-20)], ids=lambda v: str(v))
+def test_mixed_koren_tracer_matches_fp64(fct, value):
+    """One tracer step with the Koren limiter in FP32 against FP64. Face values are
+    convex combinations of the limiter's inputs, so the error is a few FP32 roundings of
+    the largest value: the bound of the mixed path, 1e-5 of it."""
+    import torch
+
+    import helpers
+    from test_gpu_parity import _tracer_inputs
+
+    g = helpers.small_grid(IMAX=20, JMAX=16, KMAX=33, DZ=300.0)
+    c = helpers.small_case(g)
+    helpers.perturb_state(c)
+    q0, q, d0, d, mflx, rhoq, GS, MAPF = _tracer_inputs(g, c)
+    if value is not None:  # single cells and a block of equal values
+        for x in (q0, q):
+            x[g.KS + 2, g.IS + 4, g.JS + 2] = value
+            x[g.KS + 19:g.KS + 25, g.IS + 1:g.IS + 6, g.JS:g.JS + 4] = value
+    dev = lambda x, t=torch.float64: torch.from_numpy(np.ravel(x, order="K").copy()).to("cuda", t)  # noqa: E731
+    out = []
+    hevi.setup(g.index_dict(), "UD3", "UD3KOREN1993")
+    try:
+        for mixed in (False, True):
+            ft = torch.float32 if mixed else torch.float64
+            x = dev(q0)
+            (hevi.ATMOS_DYN_Tinteg_tracer_rk3_mixed_dev if mixed else hevi.ATMOS_DYN_Tinteg_tracer_rk3_dev)(
+                QTRC=x, QTRC0=x, RHOQ_t=dev(rhoq, ft), DENS0=dev(d0), DENS=dev(d), mflx_hi=dev(mflx, ft),
+                num_diff=torch.zeros(3 * q0.size, dtype=ft, device="cuda"), GSQRT=dev(GS), MAPF=dev(MAPF), CDZ=g.CDZ,
+                RCDZ=g.RCDZ, RCDX=g.RCDX, RCDY=g.RCDY, BND_W=False, BND_E=False, BND_S=False, BND_N=False, dtl=2.0,
+                FLAG_FCT_TRACER=fct, FLAG_FCT_ALONG_STREAM=True)
+            hevi.check()
+            out.append(x.cpu().numpy().reshape(g.shape, order="F"))
+    finally:
+        hevi.finalize()
+    assert np.isfinite(out[1]).all()
+    emax, _ = field_errors(out[1], out[0], g)
+    assert emax <= 1e-5, emax
