@@ -209,8 +209,8 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
     }
     const int i0 = g.IS + ti * TX, j0 = g.JS + tj * TY;
     const bool col_ok = i0 + tx <= g.IE && j0 + ty <= g.JE;
-    // warps beyond the domain's edge run along, on its first halo column at most
-    // (whose DPRES the last column needs), and store nothing
+    // warps beyond the domain's edge run along and store nothing; the first halo column's
+    // forms the DPRES that the last column needs
     const int i = min(i0 + tx, g.IE + 1), j = min(j0 + ty, g.JE + 1);
     const size_t N3 = n3(g);
     const int sI = g.KA, sJ = g.KA * g.IA;
@@ -261,6 +261,15 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
 
     // this warp's column in the staged box, at the lane's level of the chunk
     const int cbox = ((ty + H) * BW + (tx + H)) * BK + KLO + lane;
+    // the column it computes on: a warp beyond the domain's edge takes the edge's, as its
+    // own may have neighbours beyond the array, where nothing (cp.async) or zero (TMA) is
+    // staged. On those its quotients left the range of the straight-line form, the Koren
+    // limiter took its general form, and the CTA waited for it: a step at 61x53x40, UD3,
+    // 281 -> 255 us, at 61x53x41, Koren, 537 -> 409 us with the levels below. FP32 without
+    // the limiter keeps its own column, 0.5% faster at 256x256x96.
+    constexpr bool EDGE_COL = sizeof(R) == 8 || S == KOREN;
+    const int crun = !EDGE_COL ? cbox
+                               : ((min(ty, g.JE - j0) + H) * BW + (min(tx, g.IE - i0) + H)) * BK + KLO + lane;
     // this column's DPRES and RT2P at level k = L-1 ([1]: at level L), and DPRES at level L
     // of its +x and +y neighbours: the tile's columns, then the +x and the +y side
     double *const dpc = sdp + w * NDP + lane, *const rtc = srp + w * NDP + lane;
@@ -409,9 +418,12 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
 #define wd_k lt[5 * NDP]
         auto chunk = [&](auto edge) {
             constexpr bool EDGE = decltype(edge)::value;
-            const double *const sDN = stg + F_DN * PL + cbox, *const sMZ = stg + F_MZ * PL + cbox;
-            const double *const sMX = stg + F_MX * PL + cbox, *const sMY = stg + F_MY * PL + cbox;
-            const double *const sPO = stg + F_RT * PL + cbox; // POTT
+            // without tensor maps, lanes above KE have levels where nothing is staged either;
+            // only the limiter minds
+            const int here = crun + (S == KOREN && LD == LD_COPY ? lev + 1 - L : 0);
+            const double *const sDN = stg + F_DN * PL + here, *const sMZ = stg + F_MZ * PL + here;
+            const double *const sMX = stg + F_MX * PL + here, *const sMY = stg + F_MY * PL + here;
+            const double *const sPO = stg + F_RT * PL + here; // POTT
             auto zf = [&](R vel, int m, const auto &v) -> R {
                 if constexpr (EDGE) return zface<S>(vel, m, KS, KE, v);
                 else return zface_in<S>(vel, m, v);

@@ -37,3 +37,12 @@ def test_split_and_marched_columns(lib, scheme, size, kmax):
         lib.ATMOS_DYN_Tstep_short_fvm_hevi(**kw, **out[-1])
     for n in out[0]:
         assert helpers.same(out[0][n], out[1][n]), n
+
+
+# tiles that reach beyond the domain, and beyond the array, by 1 to 3 columns; odd KA stages
+# with cp.async, which leaves what lies beyond the array as it was
+@pytest.mark.parametrize("kmax", [40, 41, 65])
+@pytest.mark.parametrize("size", [(5, 6), (6, 7), (7, 5), (8, 8), (33, 29)], ids=str)
+@pytest.mark.parametrize("scheme", ["UD3", "UD3KOREN1993", "UD5"])
+def test_ragged_tiles(lib, scheme, size, kmax):
+    test_split_and_marched_columns(lib, scheme, size, kmax)
