@@ -27,7 +27,6 @@
 
 namespace hevi {
 
-#ifndef HEVI_FLOAT_TU
 namespace {
 
 // staggering ids (scale_atmos_grid_cartesC_index.F90:90-101), variable ids and directions
@@ -616,6 +615,5 @@ cudaError_t launch_terrain_stage(const Grid &g, const StageArgsT<double> &a, con
     default: return cudaErrorInvalidValue;
     }
 }
-#endif // HEVI_FLOAT_TU
 
 }  // namespace hevi

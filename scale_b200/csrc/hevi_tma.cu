@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
             // box origin (0-based): level L0-4 = KST*ch - 2 (even, so its byte offset is a
             // multiple of 16), column i0-H, row j0-H
             const int x = KST * ch + (KS - 1) - KLO, y = i0 - H - 1, z = j0 - H - 1;
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            fence_proxy_async();
             mbar_expect_tx(bar, (unsigned)(NF * PL * sizeof(double)));
             for (int f = 0; f < NF; ++f) tma_load_3d(stg + f * PL, &maps.m[f], x, y, z, bar);
         } else {
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(32 * NCOL, wide_scheme(S) ? 1 : 2)
     if (LD == LD_TMA && tid == 0) {
         s_ok = 1;
         mbar_init(bar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_mbar_init();
     }
     issue(ch0);
     __syncthreads();
