@@ -517,7 +517,9 @@ int scale_hevi_persistent_grid(int *ctas);
  * tile_x x (16/tile_x); a mixed-precision ensemble has it alone (width 16 for
  * tile_x = 0). CTAs are issued in raster groups of `raster` tile rows (0: 16).
  * The shape changes the speed only: FP64 results are identical for every
- * shape; FP32 arithmetic may round differently in the two forms.
+ * shape (the tiled form's quotients of dividends under 2^-900 in magnitude
+ * may differ in the last place); FP32 arithmetic may round differently in the
+ * two forms.
  * ------------------------------------------------------------------------- */
 int scale_hevi_stage_shape(int tile_x, int raster);
 /* Autotuner of that shape. With enable != 0, the next short-step call of each

@@ -291,10 +291,10 @@ template cudaError_t launch_hevi_stage<float>(const Grid &, const Members &, con
 template cudaError_t launch_hevi_stage<double>(const Grid &, const Members &, const StageArgsT<double> &, int,
                                                StageShape, cudaStream_t, int *, bool *);
 
-// at least 10 CTAs per SM (51 registers): the loop nests are bound by load
-// latency, and unbounded they took 29-90 registers (5 CTAs per SM for the
-// largest); 512x512x128 CD4 terrain short step 81.1 -> 75.4 ms (8 CTAs 77.4,
-// 12 CTAs 78.9)
+// The loop nests of the general-metric HEVE stage. At least 10 CTAs per SM (51
+// registers): they are bound by load latency, and unbounded they took 29-90 registers
+// (5 CTAs per SM for the largest); 256x256x64 CD4 HEVE short step 10.98 -> 8.45 ms (8
+// CTAs 8.86)
 #ifndef HEVI_GCOLS_MINB
 #define HEVI_GCOLS_MINB 10
 #endif

@@ -265,7 +265,8 @@ def set_halo_exchange(fn) -> None:
 
 
 def stage_shape(tile_x: int = 0, raster: int = 0) -> None:
-    """Tile width and raster height of the stage kernel (0: defaults)."""
+    """Form and tile width (0: the tiled form where it applies, else the fused kernel's
+    default; 16, 8, 4: the fused kernel) and raster height (0: default) of the stage."""
     _check(load().scale_hevi_stage_shape(int(tile_x), int(raster)))
 
 
@@ -416,7 +417,8 @@ def persistent_wait(seconds: float, extra_arrivals: int = 0) -> None:
 
 
 def numfilter_form(tiled: bool) -> None:
-    """The filter's tiled form (True, the default) or the column kernel for one domain."""
+    """The filter's tiled form (True, the default) or the column kernel, for one domain
+    and for an ensemble."""
     _check(load().scale_hevi_numfilter_form(int(bool(tiled))))
 
 
